@@ -826,11 +826,13 @@ spk_status spk_render_denoised(spk_ctx *ctx, spk_denoiser *dn, uint32_t spp, uin
     const uint32_t w = cfg.width, h = cfg.height;
     const size_t px = static_cast<size_t>(w) * h;
     cudaSetDevice(dn->device);
-    // scratch: half A, three feature sets, three denoised images, the output
-    DN_TRY(dn->frame.ensure(px * (4 + 3 * SPK_DN_FEATURES + 3 * 4 + 4)), "frame scratch");
-    float *half_a = dn->frame.p, *feat = half_a + 4 * px, *feat_a = feat + SPK_DN_FEATURES * px,
-          *feat_b = feat_a + SPK_DN_FEATURES * px, *den = feat_b + SPK_DN_FEATURES * px, *den_a = den + 4 * px,
-          *den_b = den_a + 4 * px, *out = den_b + 4 * px;
+    // scratch: half A, three denoised images and the output (float4 records, so they come first: the buffer's
+    // start and every multiple of 16 px bytes are 16-byte aligned at any pixel count), then three feature sets
+    // (10 floats per pixel)
+    DN_TRY(dn->frame.ensure(px * (4 + 3 * 4 + 4 + 3 * SPK_DN_FEATURES)), "frame scratch");
+    float *half_a = dn->frame.p, *den = half_a + 4 * px, *den_a = den + 4 * px, *den_b = den_a + 4 * px,
+          *out = den_b + 4 * px, *feat = out + 4 * px, *feat_a = feat + SPK_DN_FEATURES * px,
+          *feat_b = feat_a + SPK_DN_FEATURES * px;
     void *fb = nullptr, *img = nullptr, *nd = nullptr, *alb = nullptr;
     const uint32_t half = spp / 2;
     if (half >= 1) {
