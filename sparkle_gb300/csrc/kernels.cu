@@ -15,7 +15,7 @@ namespace {
 template <int kMode, bool kCount>
 __global__ void __launch_bounds__(128, SPK_WALK_MIN_BLOCKS) k_trace(DevScene S, const float *__restrict__ rays, uint64_t n,
                                                   spk_hit_dev *__restrict__ hits, Counters *counters) {
-    uint32_t err = 0, done = 0;
+    uint32_t err = 0;
     TraceCounts tc;
     walk_persistent<kMode, kCount>(
         S, &counters->queue_counters[0], n, kFltMax, err, &tc,
@@ -35,9 +35,8 @@ __global__ void __launch_bounds__(128, SPK_WALK_MIN_BLOCKS) k_trace(DevScene S, 
                 out = spk_hit_dev{0.f, 0.f, 0.f, res.inst, kInvalid};
             }
             hits[q] = out;
-            ++done;
         });
-    warp_add_u64(&counters->extension_rays, done);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&counters->extension_rays, n);
     if (kCount) {
         warp_add_u64(&counters->node_visits, tc.nodes);
         warp_add_u64(&counters->tri_tests, tc.tris);

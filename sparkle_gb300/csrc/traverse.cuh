@@ -18,8 +18,8 @@
 // every box of the level; here that axis is tested as an exact containment test instead.
 //
 // The walk is a resumable state machine (Walker::step) so persistent warps can replace finished rays
-// with new ones while the others are still walking (dynamic ray fetch), and it postpones triangle groups
-// when only a few lanes of the warp have triangles to test, keeping the lanes on the same kind of work.
+// with new ones while the others are still walking (dynamic ray fetch). A persistent warp collects the triangles its
+// rays reach and tests 32 at a time, one per lane (TriangleQueue).
 #pragma once
 
 #include "device_scene.cuh"
@@ -30,35 +30,17 @@ enum : int { kTraceClosest = 0, kTraceAnyRef = 1, kTraceOcclusion = 2 };
 enum : uint32_t { kErrStackOverflow = 1u, kErrIterationBudget = 2u, kErrQueueOverflow = 4u };
 
 // Tunables (compile-time; the autotuner builds variants by defining them).
-#ifndef SPK_POSTPONE_LANES
-#define SPK_POSTPONE_LANES 8  // postpone triangle groups when fewer lanes than this want triangles
-#endif
 #ifndef SPK_REFILL_LANES
-#define SPK_REFILL_LANES 20  // persistent warps refill idle lanes once fewer than this are walking
+#define SPK_REFILL_LANES 22  // persistent warps refill idle lanes once fewer than this are walking
 #endif
-#ifndef SPK_BYTE_CONVERT_PRMT
-#define SPK_BYTE_CONVERT_PRMT 0  // 1: quantised plane bytes to float with a byte permute + add
-#endif
-#ifndef SPK_POSTPONE_INNER
-#define SPK_POSTPONE_INNER 0  // 1: also postpone inside the triangle loop as lanes drop out of it
-#endif
-#ifndef SPK_MINMAX3
-#define SPK_MINMAX3 0  // 1: slab entry/exit with three-input min/max (exact, same results)
-#endif
-#ifndef SPK_META_SIMD
-#define SPK_META_SIMD 1  // 1: the four meta bytes of a half node decoded together with 32-bit SIMD-in-register ops
-#endif
-#ifndef SPK_MT_RCP
-#define SPK_MT_RCP 1  // 1: Moller-Trumbore's 1/det as a correctly rounded reciprocal (same bits as 1.f/det)
-#endif
-#ifndef SPK_SLAB_RCP
-#define SPK_SLAB_RCP 0  // 1: the slab reciprocals as correctly rounded reciprocals (same bits as 1.f/x)
+#ifndef SPK_TAIL_STEPS
+#define SPK_TAIL_STEPS 4  // steps between the rounds of a persistent warp that has no more rays to fetch
 #endif
 #ifndef SPK_WALK_MIN_BLOCKS
 #define SPK_WALK_MIN_BLOCKS 7  // resident 128-thread blocks per SM of the closest-hit walks (72 registers)
 #endif
 #ifndef SPK_SHADOW_MIN_BLOCKS
-#define SPK_SHADOW_MIN_BLOCKS 8  // the same for the occlusion walk of the shadow stage (64 registers)
+#define SPK_SHADOW_MIN_BLOCKS 7  // the same for the occlusion walk of the shadow stage
 #endif
 #ifndef SPK_PACKET_MIN_BLOCKS
 #define SPK_PACKET_MIN_BLOCKS 8  // resident 128-thread blocks per SM the packet walk is compiled for
@@ -78,29 +60,30 @@ enum : uint32_t { kErrStackOverflow = 1u, kErrIterationBudget = 2u, kErrQueueOve
 #ifndef SPK_PACKET_SIBLINGS
 #define SPK_PACKET_SIBLINGS 4  // sibling nodes a packet tests at once (one per 8-lane group), 1..4
 #endif
-#ifndef SPK_SMEM_STACK
-#define SPK_SMEM_STACK 0  // top entries of each persistent walk's stack kept in shared memory (0: all local)
-#endif
-#ifndef SPK_STACK_REGTOP
-#define SPK_STACK_REGTOP 0  // 1: the top entry of each persistent walk's local stack cached in registers
-#endif
-
 constexpr int kStackSize = 48;
 constexpr int kWalkThreads = 128;  // threads per block of every persistent walking kernel
 constexpr uint32_t kMaxIterations = 1u << 20;
-constexpr int kPostponeLanes = SPK_POSTPONE_LANES;
 constexpr uint32_t kPacketSiblings = SPK_PACKET_SIBLINGS;
 constexpr uint32_t kPacketStack = 64;  // packet walks push up to 2 * kPacketSiblings - 1 groups per node step
 static_assert(kPacketSiblings >= 1 && kPacketSiblings <= 4, "one to four 8-lane groups");
 
-// Byte `c` of `word` as a float (exact for 0..255).
-__device__ __forceinline__ float byte_to_float(uint32_t word, int c) {
-#if SPK_BYTE_CONVERT_PRMT
-    // 0x4B0000xx is 2^23 + xx; subtracting 2^23 is exact.
-    return __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u | static_cast<uint32_t>(c))) - 8388608.0f;
-#else
-    return static_cast<float>((word >> (8 * c)) & 0xFFu);
-#endif
+// 65536 + byte `c` of `word`: the byte, times 128, added to the bits of 65536.f (whose last place is 1/128). The byte dot
+// product does it in one instruction of the FMA pipe, where a byte permute, or an extraction and a conversion, would
+// go to the ALU pipe, the walk's busiest (it also takes the slab minima and maxima).
+__device__ __forceinline__ float plane(uint32_t word, int c) {
+    return __uint_as_float(__dp4a(word, 128u << (8 * c), 0x47800000u));
+}
+// Packed single-precision fused multiply-add (the halves rounded as fmaf rounds them).
+__device__ __forceinline__ unsigned long long pack_f2(float lo, float hi) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void fma_f2(unsigned long long a, unsigned long long b, unsigned long long c, float &lo,
+                                       float &hi) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
 }
 
 struct TraceResult {
@@ -119,108 +102,138 @@ struct LevelRay {
     uint32_t oct;  // bit k set when direction component k is negative
 };
 
-// Reciprocal for the slab test; a component with |d| <= FLT_EPSILON gets +-2^100 so that
+// Reciprocal for the slab test; a component with |d| <= FLT_EPSILON gets +-2^92 so that
 // (bound - o) * inv keeps its exact sign without overflowing (an exact containment test on that axis).
+// kExact: correctly rounded (the packet walk's interval bounds carry no slack for it); otherwise the hardware's
+// approximate reciprocal (relative error <= 2^-23, part of visit_slots's slack).
+template <bool kExact>
 __device__ __forceinline__ float slab_inverse(float x) {
-#if SPK_SLAB_RCP
-    return fabsf(x) <= 1.1920928955078125e-07f ? copysignf(0x1p100f, x) : __frcp_rn(x);  // the bits of 1.f / x
-#else
-    return fabsf(x) <= 1.1920928955078125e-07f ? copysignf(0x1p100f, x) : 1.f / x;
-#endif
+    float r;
+    if (kExact) {
+        r = 1.f / x;
+    } else {
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    }
+    return fabsf(x) <= 1.1920928955078125e-07f ? copysignf(0x1p92f, x) : r;
 }
 
+template <bool kExact = false>
 __device__ __forceinline__ void setup_level(LevelRay &r, f3 o, f3 d) {
     r.o = o;
     r.d = d;
-    r.inv = mk3(slab_inverse(d.x), slab_inverse(d.y), slab_inverse(d.z));
+    r.inv = mk3(slab_inverse<kExact>(d.x), slab_inverse<kExact>(d.y), slab_inverse<kExact>(d.z));
     r.oct = (signbit(d.x) ? 1u : 0u) | (signbit(d.y) ? 2u : 0u) | (signbit(d.z) ? 4u : 0u);
 }
 
 // Upper bound on the t a box may start at and still hold a hit closer than `best` (in world-t terms).
-__device__ __forceinline__ float prune_limit(float best, f3 wo, f3 wd, float scene_abs_x) {
+__device__ __forceinline__ float prune_limit(float best, float wox, float wdx, float scene_abs_x) {
     if (!(best < kFltMax)) return kFltMax;
-    const float ax = fabsf(wd.x);
-    const float slack = ax > 0.f ? (fabsf(wo.x) + scene_abs_x) * 0x1p-18f / ax : kFltMax;
+    float r;  // 1 / |wdx| within 2^-23; infinite below 2^-126, which leaves the limit open
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(wdx)));
+    const float slack = (fabsf(wox) + scene_abs_x) * 0x1.00001p-18f * r;
     const float lim = best * (1.f + 0x1p-14f) + slack;
     return isfinite(lim) ? lim : kFltMax;
 }
 
-// Slab test of the 8 children of one wide node; returns the next node group (inner children, permuted
-// slot bits 24..31 + imask in bits 0..7) and triangle group (leaf items, bits 0..23). The ray's own octant
-// picks each slab's near and far planes; `order` (an octant) permutes the inner children's bits, which sets
-// the visiting order (a single-ray walk passes its own octant, a packet one octant shared by its lanes).
-// Three-input max / min (PTX max.f32 / min.f32 with three operands): the same value as the two-input
-// forms applied in turn, NaN operands ignored.
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-__device__ __forceinline__ float min3f(float a, float b, float c) {
-    float d;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
+// Slots of a node in a ray's visiting order: first[oct][mask] is the slot s of `mask` (a non-zero set of the 8
+// slots) with the smallest s ^ oct, the child nearest along a ray of octant `oct`.
+struct SlotOrder {
+    uint8_t first[8][256];
+    constexpr SlotOrder() : first() {
+        for (int oct = 0; oct < 8; ++oct)
+            for (int mask = 1; mask < 256; ++mask)
+                for (int k = 7; k >= 0; --k)
+                    if ((mask >> (k ^ oct)) & 1) first[oct][mask] = static_cast<uint8_t>(k ^ oct);
+    }
+};
+static __device__ const SlotOrder kSlotOrder{};
+
+// Slot mask with slot s moved to bit s ^ oct (the packet walk's groups: lowest bit first is the visiting order).
+__device__ __forceinline__ uint32_t order_slots(uint32_t mask, uint32_t oct) {
+    if (oct & 1u) mask = ((mask & 0x55u) << 1) | ((mask >> 1) & 0x55u);
+    if (oct & 2u) mask = ((mask & 0x33u) << 2) | ((mask >> 2) & 0x33u);
+    if (oct & 4u) mask = ((mask & 0x0Fu) << 4) | (mask >> 4);
+    return mask;
 }
 
-__device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint32_t idx, const LevelRay &r,
-                                           uint32_t order, float tmax, uint2 &ngroup, uint2 &tgroup) {
+// What a ray's slab tests found in a node.
+struct NodeHits {
+    uint32_t child_base, item_base;
+    uint32_t imask;       // slots that hold inner nodes
+    uint32_t hit;         // slots whose box the ray enters
+    uint32_t meta[2];     // per slot: leaf items (unary count << 5 | first item) or an inner child's marker
+};
+
+// Slab test of the 8 children of node `idx` against one ray, in pairs of children (packed multiply-adds).
+//
+// Bound: instruction issue and the ALU pipe, which runs at half the issue rate. Per visit of random nodes (a loop of
+// visits, counted by ncu): 277 warp instructions of which 159 on the ALU pipe with the byte planes converted one by one,
+// scalar or packed near / far, and every hit child's item bits assembled here; 194 and 81 now: the planes come from byte
+// dot products (FMA pipe), the packed operands are two children's (which needs no register moves), and only the slot
+// mask is built here (leaf items are decoded by the few rays that reach a leaf).
+//
+// A child passes whenever its quantised box is entered within [0, tmax] in exact arithmetic. Per axis, with
+// inv = (1 / d)(1 + e), |e| <= 2^-23, the plane at byte q is at t = q a + o, a = scale * inv, o = (p - r.o) * inv,
+// evaluated as fma(65536 + q, a, o -+ slack - 65536 a). Errors: |o| (2^-22 from o itself, 3 * 2^-24 from the three later
+// roundings) and |a| (2 * 2^-8 from the roundings of o - 65536 a and its slack, below 2^-14 the rest), within the slack
+// of 2^-20 |o| + 2^-6 |a|. The slack also covers the rounding of the plain fma(q, a, o), so every box that form lets
+// pass passes here. (|o| is cut at 2^100 in the slack so that an overflowing o still misses: inf - inf would pass.)
+__device__ __forceinline__ NodeHits visit_slots(const uint4 *__restrict__ nodes, uint32_t idx, const LevelRay &r,
+                                                float tmax) {
     const uint4 *np = nodes + static_cast<size_t>(idx) * 5;
     const uint4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
-    const float sx = __uint_as_float((n0.w & 0xFFu) << 23);
-    const float sy = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23);
-    const float sz = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23);
-    const float ax = sx * r.inv.x, ay = sy * r.inv.y, az = sz * r.inv.z;
-    const float ox = (__uint_as_float(n0.x) - r.o.x) * r.inv.x;
-    const float oy = (__uint_as_float(n0.y) - r.o.y) * r.inv.y;
-    const float oz = (__uint_as_float(n0.z) - r.o.z) * r.inv.z;
-    uint32_t hitmask = 0;
+    float a[3], near_o[3], far_o[3];
+    const float p[3] = {__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)};
+    const float ro[3] = {r.o.x, r.o.y, r.o.z}, ri[3] = {r.inv.x, r.inv.y, r.inv.z};
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t meta4 = h ? n1.w : n1.z;
-        const uint32_t lox = h ? n2.y : n2.x, loy = h ? n2.w : n2.z, loz = h ? n3.y : n3.x;
-        const uint32_t hix = h ? n3.w : n3.z, hiy = h ? n4.y : n4.x, hiz = h ? n4.w : n4.z;
-        const uint32_t nx = (r.oct & 1u) ? hix : lox, fx = (r.oct & 1u) ? lox : hix;
-        const uint32_t ny = (r.oct & 2u) ? hiy : loy, fy = (r.oct & 2u) ? loy : hiy;
-        const uint32_t nz = (r.oct & 4u) ? hiz : loz, fz = (r.oct & 4u) ? loz : hiz;
-#if SPK_META_SIMD
-        // Per byte: an inner child has bits 3 and 4 of its meta set; its slot bit is xor-ed with the ray's
-        // octant. bit4 = the hit-mask bit index of each child, bits4 = the bits it sets there (0 for an
-        // empty slot, whose meta byte is 0, so empty slots need no test of their own).
-        const uint32_t inner4 = (meta4 & (meta4 << 1)) & 0x10101010u;
-        const uint32_t bit4 = (meta4 ^ ((inner4 >> 4) * order)) & 0x1F1F1F1Fu;
-        const uint32_t bits4 = (meta4 >> 5) & 0x07070707u;
-#endif
+    for (int k = 0; k < 3; ++k) {
+        a[k] = __uint_as_float(((n0.w >> (8 * k)) & 0xFFu) << 23) * ri[k];
+        const float o = (p[k] - ro[k]) * ri[k];
+        const float base = fmaf(-65536.f, a[k], o);
+        const float slack = fmaf(fminf(fabsf(o), 0x1p100f), 0x1p-20f, fabsf(a[k]) * 0x1p-6f);
+        near_o[k] = base - slack;
+        far_o[k] = base + slack;
+    }
+    NodeHits h{n1.x, n1.y, n0.w >> 24, 0u, {n1.z, n1.w}};
+    const uint32_t lo[3][2] = {{n2.x, n2.y}, {n2.z, n2.w}, {n3.x, n3.y}};
+    const uint32_t hi[3][2] = {{n3.z, n3.w}, {n4.x, n4.y}, {n4.z, n4.w}};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-#if !SPK_META_SIMD
-            const uint32_t m = (meta4 >> (8 * c)) & 0xFFu;
-#endif
-            const float tnx = fmaf(byte_to_float(nx, c), ax, ox);
-            const float tny = fmaf(byte_to_float(ny, c), ay, oy);
-            const float tnz = fmaf(byte_to_float(nz, c), az, oz);
-            const float tfx = fmaf(byte_to_float(fx, c), ax, ox);
-            const float tfy = fmaf(byte_to_float(fy, c), ay, oy);
-            const float tfz = fmaf(byte_to_float(fz, c), az, oz);
-#if SPK_MINMAX3
-            const float t0 = max3f(tnx, tny, fmaxf(tnz, 0.f));
-            const float t1 = min3f(tfx, tfy, fminf(tfz, tmax));
-#else
-            const float t0 = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, 0.f));
-            const float t1 = fminf(fminf(tfx, tfy), fminf(tfz, tmax));
-#endif
-#if SPK_META_SIMD
-            if (t0 <= t1) hitmask |= __byte_perm(bits4, 0u, 0x4440u | c) << __byte_perm(bit4, 0u, 0x4440u | c);
-#else
-            if (m != 0u && t0 <= t1) {
-                uint32_t bit = m & 0x1Fu;
-                if ((m & 0x18u) == 0x18u) bit ^= order;
-                hitmask |= ((m >> 5) & 7u) << bit;
+    for (int half = 0; half < 2; ++half) {
+        uint32_t nw[3], fw[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const bool neg = (r.oct >> k) & 1u;
+            nw[k] = neg ? hi[k][half] : lo[k][half];
+            fw[k] = neg ? lo[k][half] : hi[k][half];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+            float tn[3][2], tf[3][2];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const unsigned long long a2 = pack_f2(a[k], a[k]);
+                fma_f2(pack_f2(plane(nw[k], c), plane(nw[k], c + 1)), a2, pack_f2(near_o[k], near_o[k]), tn[k][0], tn[k][1]);
+                fma_f2(pack_f2(plane(fw[k], c), plane(fw[k], c + 1)), a2, pack_f2(far_o[k], far_o[k]), tf[k][0], tf[k][1]);
             }
-#endif
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float t0 = fmaxf(fmaxf(tn[0][e], tn[1][e]), fmaxf(tn[2][e], 0.f));
+                const float t1 = fminf(fminf(tf[0][e], tf[1][e]), fminf(tf[2][e], tmax));
+                if (t0 <= t1) h.hit |= 1u << (4 * half + c + e);
+            }
         }
     }
-    ngroup = make_uint2(n1.x, (hitmask & 0xFF000000u) | (n0.w >> 24));
-    tgroup = make_uint2(n1.y, hitmask & 0x00FFFFFFu);
+    return h;
+}
+
+// The triangle (or TLAS item) bits of the leaf slots `leaf` of a node.
+__device__ __forceinline__ uint32_t leaf_items(uint32_t leaf, const uint32_t (&meta)[2]) {
+    uint32_t bits = 0u;
+    for (; leaf != 0u; leaf &= leaf - 1u) {
+        const uint32_t m = __byte_perm(meta[0], meta[1], __ffs(leaf) - 1);
+        bits |= ((m >> 5) & 7u) << (m & 31u);
+    }
+    return bits;
 }
 
 // Möller–Trumbore (MeshRenderProxy.cpp:128-194) of triangle record `idx` in the level ray's (the instance's
@@ -234,11 +247,7 @@ __device__ __forceinline__ bool triangle_hit(const float4 *__restrict__ tris, ui
     const float det = dot3(e1, h);
     if (fabsf(det) < kEps) return false;
     const f3 s = ray.o - p0;
-#if SPK_MT_RCP
-    const float f = __frcp_rn(det);
-#else
-    const float f = 1.f / det;
-#endif
+    const float f = __frcp_rn(det);  // the bits of 1.f / det
     u = f * dot3(s, h);
     if (u < 0.f || u > 1.f) return false;
     const f3 q = cross(s, e1);
@@ -269,106 +278,71 @@ __device__ __forceinline__ bool sphere_hit(const DevInstance &I, f3 wo, f3 wd, f
     return true;
 }
 
-// Traversal stacks. Walker::push / pop address entry `i` (0 = bottom) of the current ray's stack.
-// LocalStack: the whole stack in local memory (one-thread walks).
+// The traversal stack of one ray in local memory (it hits in L1; the stack is about 1% of a walk's instructions).
 struct LocalStack {
     uint2 e[kStackSize];
-    __device__ __forceinline__ void reset() {}
     __device__ __forceinline__ void put(int i, uint2 v) { e[i] = v; }
     __device__ __forceinline__ uint2 take(int i) { return e[i]; }
 };
 
-// SharedRingStack: the top K entries in a per-thread ring of shared memory, deeper entries in local memory.
-// Invariant: entries [max(0, sp - K), sp) are in the ring, entry i in slot i mod K; pushing entry i >= K
-// first moves entry i - K out to local memory, popping it brings entry i - K back into the freed slot. The
-// ring is a column of the block's array (slot k of thread t at k * kWalkThreads + t): the 16 lanes of a
-// half-warp touch 16 consecutive 8-byte words whatever their depths, so accesses are free of bank conflicts.
-template <int K>
-struct SharedRingStack {
-    static_assert(K > 0 && (K & (K - 1)) == 0 && K < kStackSize, "ring size: a power of two below the stack size");
-    uint2 *ring;  // this thread's slot 0
-    uint2 spill[kStackSize - K];
-    __device__ __forceinline__ void reset() {}
-    __device__ __forceinline__ void put(int i, uint2 v) {
-        uint2 *slot = ring + (i & (K - 1)) * kWalkThreads;
-        if (i >= K) spill[i - K] = *slot;
-        *slot = v;
-    }
-    __device__ __forceinline__ uint2 take(int i) {
-        uint2 *slot = ring + (i & (K - 1)) * kWalkThreads;
-        const uint2 v = *slot;
-        if (i >= K) *slot = spill[i - K];
-        return v;
-    }
-};
-
-// RegTopStack: a local stack whose top entry may live in registers instead (`cached`): a push moves the
-// cached entry out to local memory and caches the new one, a pop returns the cached entry when there is
-// one, so a push followed by its pop touches no memory.
-struct RegTopStack {
-    uint2 top;
-    bool cached = false;
-    uint2 e[kStackSize];
-    // A walk that ended early (an occlusion hit) may leave entries behind, the top one cached.
-    __device__ __forceinline__ void reset() { cached = false; }
-    __device__ __forceinline__ void put(int i, uint2 v) {
-        if (cached) e[i - 1] = top;
-        top = v;
-        cached = true;
-    }
-    __device__ __forceinline__ uint2 take(int i) {
-        if (cached) {
-            cached = false;
-            return top;
-        }
-        return e[i];
-    }
-};
-
 // True when a hit at world t `t` on (inst, face) replaces `best`: a smaller t, or an exact tie on a smaller
-// (instance, face).
+// (instance, face). The reference keeps the first of equal t (IntersectionCandidate::IsCloserHit is a strict <),
+// which depends on the visit order; this rule makes every hit independent of scheduling.
 __device__ __forceinline__ bool closer_hit(const TraceResult &best, float t, uint32_t inst, uint32_t face) {
     if (t < best.t) return true;
     return t == best.t && (inst < best.inst || (inst == best.inst && face < best.face));
 }
 
-// Resumable two-level walk of one ray. init() starts it; step() advances by one node visit plus the
-// triangle tests it enables and returns true when the walk is over (result in `best`).
-template <int kMode, bool kCount>
+// Where a walk keeps its world ray. A one-thread walk: registers. A persistent walk: a column of the block's
+// shared memory (component k of thread t at [k][t]: any set of lanes reads its own or other lanes' rays without
+// bank conflicts), so that other lanes of the warp can test its triangles (TriangleQueue).
+struct RegWorld {
+    f3 ro, rd;
+    __device__ __forceinline__ void set(f3 a, f3 b) {
+        ro = a;
+        rd = b;
+    }
+    __device__ __forceinline__ f3 o() const { return ro; }
+    __device__ __forceinline__ f3 d() const { return rd; }
+};
+struct SharedWorld {
+    float *w;  // component 0 of this thread
+    __device__ __forceinline__ void set(f3 a, f3 b) {
+        const float v[6] = {a.x, a.y, a.z, b.x, b.y, b.z};
+#pragma unroll
+        for (int k = 0; k < 6; ++k) w[k * kWalkThreads] = v[k];
+    }
+    __device__ __forceinline__ f3 o() const { return mk3(w[0], w[kWalkThreads], w[2 * kWalkThreads]); }
+    __device__ __forceinline__ f3 d() const {
+        return mk3(w[3 * kWalkThreads], w[4 * kWalkThreads], w[5 * kWalkThreads]);
+    }
+};
+
+// Resumable two-level walk of one ray. init() starts it; step() advances by one node visit and returns true when
+// the walk is over (result in `best`).
+template <int kMode, bool kCount, class World>
 struct Walker {
-    f3 wo, wd;
+    World world;
     LevelRay ray;
-    uint2 ngroup, tgroup;
-    int sp, blas_sp;
+    uint2 ngroup;
+    int sp;
+    int blas_sp;  // stack height the BLAS was entered at; -1 at the TLAS level, -2 there before `ray` is the world ray again
     uint32_t cur_inst;
-    uint32_t iter, budget;
-    bool in_blas;
-    float tmax_box, tmax_occl;
+    uint32_t steps_left;
+    float tmax_box;
     TraceResult best;
 
     // `root` is the TLAS root node of the ray's scene (S.tlas_root for a single-scene context).
     __device__ __forceinline__ void init(const DevScene &S, uint32_t root, f3 o, f3 d, float tmax) {
-        wo = o;
-        wd = d;
+        world.set(o, d);
         setup_level(ray, o, d);
         ngroup = make_uint2(root, root == kInvalid ? 0u : (1u << 24));
-        tgroup = make_uint2(0u, 0u);
         sp = 0;
-        blas_sp = 0;
+        blas_sp = -1;
         cur_inst = 0;
-        iter = 0;
-        budget = S.walk_budget ? S.walk_budget : kMaxIterations;
-        in_blas = false;
-        tmax_occl = tmax;
+        steps_left = S.walk_budget ? S.walk_budget : kMaxIterations;
         tmax_box = (kMode == kTraceOcclusion) ? tmax : kFltMax;
         best = TraceResult{kFltMax, 0.f, 0.f, kInvalid, kInvalid};
-    }
-
-    // Candidate acceptance. The reference keeps the first of equal t (IntersectionCandidate::IsCloserHit is
-    // a strict <), which depends on the visit order; this walk's order depends on warp composition, so an
-    // exact tie goes to the smaller (instance, face) instead, making every hit independent of scheduling.
-    __device__ __forceinline__ bool closer(float t, uint32_t inst, uint32_t face) const {
-        return closer_hit(best, t, inst, face);
     }
 
     template <class Stack>
@@ -380,174 +354,303 @@ struct Walker {
         }
     }
 
+    // Instances and spheres of a TLAS leaf group, until one opens a BLAS. True: an any-hit walk is over.
     template <class Stack>
-    __device__ __forceinline__ bool step(const DevScene &S, Stack &stack, uint32_t &err, TraceCounts *counts) {
-        if (++iter > budget) {
-            err |= kErrIterationBudget;
-            return true;
-        }
-        if (ngroup.y > 0x00FFFFFFu) {
-            const uint32_t bit = __ffs(ngroup.y >> 24) - 1;
-            ngroup.y &= ~(1u << (bit + 24));
-            const uint32_t slot = bit ^ ray.oct;
-            const uint32_t node_idx = ngroup.x + __popc(ngroup.y & 0xFFu & ((1u << slot) - 1u));
-            if (ngroup.y > 0x00FFFFFFu) push(stack, ngroup, err);
-            visit_node(S.nodes, node_idx, ray, ray.oct, tmax_box, ngroup, tgroup);
-            if (kCount) ++counts->nodes;
-            // Triangle postponing: when few lanes have triangles, keep walking nodes and test them later.
-            const uint32_t want = __ballot_sync(__activemask(), tgroup.y != 0u);
-            if (tgroup.y != 0u && ngroup.y > 0x00FFFFFFu && __popc(want) < kPostponeLanes) {
-                push(stack, tgroup, err);
-                tgroup.y = 0u;
-            }
-        } else {
-            tgroup = ngroup;
-            ngroup = make_uint2(0u, 0u);
-        }
+    __device__ __forceinline__ bool items(const DevScene &S, Stack &stack, uint2 tgroup, uint32_t &err) {
         while (tgroup.y != 0u) {
-#if SPK_POSTPONE_INNER
-            // Lanes drop out of this loop as their triangles run out; once too few are left, the rest park
-            // their remaining triangles and rejoin the node walk (only when a node visit is pending, so
-            // the parked group cannot come straight back).
-            if (in_blas && ngroup.y > 0x00FFFFFFu && __popc(__activemask()) < kPostponeLanes) {
-                push(stack, tgroup, err);
-                tgroup.y = 0u;
-                break;
-            }
-#endif
             const uint32_t k = __ffs(tgroup.y) - 1;
             tgroup.y &= tgroup.y - 1u;
-            const uint32_t idx = tgroup.x + k;
-            if (in_blas) {
-                if (kCount) ++counts->tris;
-                float t, u, v;
-                uint32_t face;
-                if (!triangle_hit(S.tris, idx, ray, t, u, v, face)) continue;
+            const uint32_t inst = __ldg(S.tlas_items + tgroup.x + k);
+            const DevInstance &I = S.instances[inst];
+            if (I.type == 1u) {
+                // SphereRenderProxy::IntersectInternal (SphereRenderProxy.cpp:5-38), world space: sphere_hit's
+                // test, written out so the any-hit modes stop before the square root.
+                const f3 wo = world.o(), wd = world.d();
+                const f3 center = mk3(I.m[3], I.m[7], I.m[11]);
+                const f3 co = wo - center;
+                const float half_b = dot3(wd, co);
+                const float c = sqnorm(co) - I.radius * I.radius;
+                const float disc = half_b * half_b - 1.f * c;
+                if (disc < 0.f) continue;
                 if (kMode == kTraceAnyRef) {
-                    best.inst = cur_inst;
+                    best.inst = inst;
                     return true;
                 }
+                const float sq = sqrtf(disc);
+                const float t = (-half_b + (c >= 0.f ? -sq : sq)) / 1.f;
                 if (kMode == kTraceOcclusion) {
-                    if (t < tmax_occl) {
-                        best.inst = cur_inst;
+                    if (t > kEps && t < tmax_box) {
+                        best.inst = inst;
                         return true;
                     }
                     continue;
                 }
-                const float wt = world_t(S.instances[cur_inst], ray, t, wo, wd);
-                if (wt > 0.f && closer(wt, cur_inst, face)) {
-                    best.t = wt;
-                    best.u = u;
-                    best.v = v;
-                    best.inst = cur_inst;
-                    best.face = face;
-                    tmax_box = prune_limit(best.t, wo, wd, S.scene_abs_x);
+                if (t > 0.f && closer_hit(best, t, inst, kInvalid)) {
+                    best = TraceResult{t, 0.f, 0.f, inst, kInvalid};
+                    tmax_box = prune_limit(best.t, wo.x, wd.x, S.scene_abs_x);
                 }
-            } else {
-                const uint32_t inst = __ldg(S.tlas_items + idx);
-                const DevInstance &I = S.instances[inst];
-                if (I.type == 1u) {
-                    // SphereRenderProxy::IntersectInternal (SphereRenderProxy.cpp:5-38), world space: sphere_hit's
-                    // test, written out so the any-hit modes stop before the square root.
-                    const f3 center = mk3(I.m[3], I.m[7], I.m[11]);
-                    const f3 co = wo - center;
-                    const float half_b = dot3(wd, co);
-                    const float c = sqnorm(co) - I.radius * I.radius;
-                    const float disc = half_b * half_b - 1.f * c;
-                    if (disc < 0.f) continue;
-                    if (kMode == kTraceAnyRef) {
-                        best.inst = inst;
-                        return true;
-                    }
-                    const float sq = sqrtf(disc);
-                    const float t = (-half_b + (c >= 0.f ? -sq : sq)) / 1.f;
-                    if (kMode == kTraceOcclusion) {
-                        if (t > kEps && t < tmax_occl) {
-                            best.inst = inst;
-                            return true;
-                        }
-                        continue;
-                    }
-                    if (t > 0.f && closer(t, inst, kInvalid)) {
-                        best.t = t;
-                        best.u = 0.f;
-                        best.v = 0.f;
-                        best.inst = inst;
-                        best.face = kInvalid;
-                        tmax_box = prune_limit(best.t, wo, wd, S.scene_abs_x);
-                    }
-                } else if (I.blas_root != kInvalid) {
-                    // Enter the BLAS: park the rest of this TLAS level on the stack.
-                    if (tgroup.y != 0u) push(stack, tgroup, err);
-                    if (ngroup.y > 0x00FFFFFFu) push(stack, ngroup, err);
-                    blas_sp = sp;
-                    in_blas = true;
-                    cur_inst = inst;
-                    setup_level(ray, xform_point(I.minv, wo), xform_dir(I.minv, wd));
-                    ngroup = make_uint2(I.blas_root, 1u << 24);
-                    tgroup.y = 0u;
-                    break;
-                }
+            } else if (I.blas_root != kInvalid) {
+                // Enter the BLAS: park the rest of this TLAS level on the stack.
+                if (tgroup.y != 0u) push(stack, tgroup, err);
+                if (ngroup.y > 0x00FFFFFFu) push(stack, ngroup, err);
+                blas_sp = sp;
+                cur_inst = inst;
+                setup_level(ray, xform_point(I.minv, world.o()), xform_dir(I.minv, world.d()));
+                ngroup = make_uint2(I.blas_root, 1u << 24);
+                tgroup.y = 0u;
             }
         }
-        if (ngroup.y <= 0x00FFFFFFu) {
-            if (in_blas && sp == blas_sp) {
-                in_blas = false;
-                setup_level(ray, wo, wd);
+        return false;
+    }
+
+    // `leaves(item_base, slots, meta)` and `group(tgroup)` take the triangles of the leaf slots reached in a node, and
+    // of a group that came back from the stack; either returns true when a hit ends the walk.
+    template <class Stack, class Leaves, class Group>
+    __device__ __forceinline__ bool step(const DevScene &S, Stack &stack, uint32_t &err, TraceCounts *counts,
+                                         Leaves &&leaves, Group &&group) {
+        if (steps_left-- == 0u) {
+            err |= kErrIterationBudget;
+            return true;
+        }
+        uint2 tgroup = make_uint2(0u, 0u);  // TLAS items
+        if (ngroup.y > 0x00FFFFFFu) {
+            const uint32_t slot = __ldg(&kSlotOrder.first[ray.oct][ngroup.y >> 24]);
+            ngroup.y &= ~(1u << (slot + 24));
+            const uint32_t node_idx = ngroup.x + __popc(ngroup.y & 0xFFu & ((1u << slot) - 1u));
+            if (ngroup.y > 0x00FFFFFFu) push(stack, ngroup, err);
+            const NodeHits h = visit_slots(S.nodes, node_idx, ray, tmax_box);
+            ngroup = make_uint2(h.child_base, ((h.hit & h.imask) << 24) | h.imask);
+            const uint32_t leaf = h.hit & ~h.imask;
+            if (kCount) ++counts->nodes;
+            if (leaf != 0u) {
+                if (blas_sp >= 0) {
+                    if (kCount) counts->tris += __popc(leaf_items(leaf, h.meta));
+                    if (leaves(h.item_base, leaf, h.meta)) return true;
+                } else {
+                    tgroup = make_uint2(h.item_base, leaf_items(leaf, h.meta));
+                }
             }
+        } else {
+            tgroup = ngroup;
+            ngroup = make_uint2(0u, 0u);
+            if (blas_sp >= 0) {
+                if (group(tgroup)) return true;
+                tgroup.y = 0u;
+            }
+        }
+        if (tgroup.y != 0u && items(S, stack, tgroup, err)) return true;
+        if (ngroup.y <= 0x00FFFFFFu) {
             if (sp == 0) return true;
+            if (sp == blas_sp) blas_sp = -2;
             ngroup = stack.take(--sp);
+            if (blas_sp == -2 && ngroup.y > 0x00FFFFFFu) {
+                setup_level(ray, world.o(), world.d());
+                blas_sp = -1;
+            }
         }
         return false;
     }
 };
 
-// Whole walk of one ray by one thread (no lane refill).
+// Whole walk of one ray by one thread, its triangles tested as they are reached.
 template <int kMode, bool kCount = false>
 __device__ __forceinline__ TraceResult trace_ray(const DevScene &S, f3 wo, f3 wd, float tmax_occl, uint32_t &err,
                                                  TraceCounts *counts = nullptr) {
     LocalStack stack;
-    Walker<kMode, kCount> w;
+    Walker<kMode, kCount, RegWorld> w;
     w.init(S, S.tlas_root, wo, wd, tmax_occl);
-    while (!w.step(S, stack, err, counts)) {
+    auto group = [&](uint2 tg) {
+        while (tg.y != 0u) {
+            const uint32_t idx = tg.x + __ffs(tg.y) - 1;
+            tg.y &= tg.y - 1u;
+            float t, u, v;
+            uint32_t face;
+            if (!triangle_hit(S.tris, idx, w.ray, t, u, v, face)) continue;
+            if (kMode == kTraceAnyRef || (kMode == kTraceOcclusion && t < tmax_occl)) {
+                w.best.inst = w.cur_inst;
+                return true;
+            }
+            if (kMode == kTraceOcclusion) continue;
+            const float wt = world_t(S.instances[w.cur_inst], w.ray, t, wo, wd);
+            if (wt > 0.f && closer_hit(w.best, wt, w.cur_inst, face)) {
+                w.best = TraceResult{wt, u, v, w.cur_inst, face};
+                w.tmax_box = prune_limit(wt, wo.x, wd.x, S.scene_abs_x);
+            }
+        }
+        return false;
+    };
+    auto leaves = [&](uint32_t base, uint32_t slots, const uint32_t (&meta)[2]) {
+        return group(make_uint2(base, leaf_items(slots, meta)));
+    };
+    while (!w.step(S, stack, err, counts, leaves, group)) {
     }
     return w.best;
 }
+
+// The triangles a warp's rays have reached and not tested yet: (triangle, instance) pairs with the lane that owns
+// the ray. Tested in the lane that reached them, triangles ran at 3.2 of 32 lanes (secondary rays of the 1024^2
+// terrain: 2 warp executions per ray, 30% of the walk's instructions); queued, a round tests 32 pairs with 26 lanes on
+// average: 550 -> 400 warp instructions per ray over the whole walk. Queueing groups instead of triangles saves the
+// writes but costs a scan per round (+4% instructions).
+constexpr uint32_t kQueueCap = 64;  // a round leaves fewer than 32, a step adds about 8 (what does not fit goes to the stack)
+struct TriangleQueue {
+    uint2 pair[kQueueCap];      // triangle record, instance
+    uint8_t owner[kQueueCap];
+    uint32_t count;             // pairs handed a place; those past kQueueCap were not stored
+    uint32_t pad;
+};
 
 // Persistent walk over a work list: each warp pulls batches of items from `cursor` and refills lanes whose
 // ray has finished once fewer than `kRefillLanes` lanes are still walking. `fetch(i, o, d, tmax)` loads item
 // i's ray (tmax starts at the call's `tmax`; an occlusion walk may lower it per ray) and returns the TLAS
 // root of its scene; `finish(i, result)` stores its result. Every lane of every warp of the block must call
-// this, and the block must have kWalkThreads threads (the shared stack rings are laid out for that many).
+// this, and the block must have kWalkThreads threads (the shared memory is laid out for that many).
+//
+// A step visits one node per walking lane and queues the triangles of the leaves it reaches; once 32 pairs are
+// queued the whole warp tests them, lane i pair i, with the owner's world ray from shared memory taken into the
+// pair's instance space (the same operations as at the BLAS entry, so the same bits). A hit goes back to its
+// owner, whose best t then prunes as before: a few steps later than if tested at once, which adds node visits (+1.6%)
+// but cannot change a result. When fewer than kRefillLanes lanes walk, every pair is tested, the walks that are over
+// store their results, and idle lanes are refilled (22: 16 and 26 are 2% slower). 72 registers (7 blocks per SM) hold a
+// walk without touching local memory in the node visits; more state in shared memory instead (8 blocks) takes L1 from
+// the nodes: measured even.
 constexpr int kRefillLanes = SPK_REFILL_LANES;
+constexpr uint32_t kTailSteps = SPK_TAIL_STEPS;
 
 template <int kMode, bool kCount, class Fetch, class Finish>
 __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long long *cursor, unsigned long long n,
                                                 float tmax, uint32_t &err, TraceCounts *counts, Fetch &&fetch,
                                                 Finish &&finish) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    __shared__ float world[6 * kWalkThreads];
+    __shared__ TriangleQueue queues[kWalkThreads / 32];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
-#if SPK_SMEM_STACK > 0
-    __shared__ uint2 rings[SPK_SMEM_STACK * kWalkThreads];
-    SharedRingStack<SPK_SMEM_STACK> stack;
-    stack.ring = rings + threadIdx.x;
-#elif SPK_STACK_REGTOP
-    RegTopStack stack;
-#else
+    TriangleQueue &Q = queues[threadIdx.x >> 5];
     LocalStack stack;
-#endif
-    Walker<kMode, kCount> w;
-    bool active = false, exhausted = false;
+    Walker<kMode, kCount, SharedWorld> w;
+    w.world.w = world + threadIdx.x;
+    bool walking = false, over = false;  // over: the walk has ended, its pairs may still be queued
+    bool exhausted = false;
+    uint32_t tail_steps = 0;
     unsigned long long item = 0;
+    if (lane == 0) Q.count = 0u;
+    __syncwarp();
+
+    // Queues `cnt` consecutive triangles (at most 3) of this lane's ray from record `first` on; returns how many found
+    // no room.
+    auto enqueue = [&](uint32_t first, uint32_t cnt) {
+        const uint32_t pos = atomicAdd(&Q.count, cnt);
+#pragma unroll
+        for (uint32_t k = 0; k < 3; ++k) {
+            if (k < cnt && pos + k < kQueueCap) {
+                Q.pair[pos + k] = make_uint2(first + k, w.cur_inst);
+                Q.owner[pos + k] = static_cast<uint8_t>(lane);
+            }
+        }
+        return pos + cnt > kQueueCap ? min(pos + cnt - kQueueCap, cnt) : 0u;
+    };
+    // What does not fit goes back to the stack.
+    auto leaves = [&](uint32_t base, uint32_t slots, const uint32_t (&meta)[2]) {
+        uint32_t left = 0u;
+        for (; slots != 0u; slots &= slots - 1u) {
+            const uint32_t m = __byte_perm(meta[0], meta[1], __ffs(slots) - 1);
+            const uint32_t at = m & 31u, cnt = __popc(m & 0xE0u);
+            const uint32_t rest = enqueue(base + at, cnt);
+            if (rest != 0u) left |= ((1u << rest) - 1u) << (at + cnt - rest);
+        }
+        if (left != 0u) w.push(stack, make_uint2(base, left), err);
+        return false;
+    };
+    auto group = [&](uint2 tg) {
+        while (tg.y != 0u) {
+            const uint32_t k = __ffs(tg.y) - 1;
+            if (enqueue(tg.x + k, 1u) != 0u) {
+                w.push(stack, tg, err);
+                break;
+            }
+            tg.y &= tg.y - 1u;
+        }
+        return false;
+    };
+    // One round: lane i tests pair i (of `cnt`); hits go to their owners; the pairs past 32 move to the front.
+    auto round = [&](uint32_t cnt) {
+        bool hit = false;
+        float t = 0.f, u = 0.f, v = 0.f;
+        uint32_t face = kInvalid, own = lane, inst = kInvalid;
+        if (lane < cnt) {
+            const uint2 e = Q.pair[lane];
+            own = Q.owner[lane];
+            inst = e.y;
+            const SharedWorld ow{world + (threadIdx.x & ~31u) + own};
+            const DevInstance &I = S.instances[inst];
+            const f3 wo = ow.o(), wd = ow.d();
+            LevelRay r;
+            r.o = xform_point(I.minv, wo);
+            r.d = xform_dir(I.minv, wd);
+            hit = triangle_hit(S.tris, e.x, r, t, u, v, face);
+            if (kMode == kTraceClosest && hit) {
+                t = world_t(I, r, t, wo, wd);
+                hit = t > 0.f;
+            }
+        }
+        if (kMode == kTraceClosest) {
+            bool closer = false;
+            for (uint32_t m = __ballot_sync(kAll, hit); m != 0u; m &= m - 1u) {
+                const int src = __ffs(m) - 1;
+                const uint32_t o = __shfl_sync(kAll, own, src);
+                const TraceResult c{__shfl_sync(kAll, t, src), __shfl_sync(kAll, u, src), __shfl_sync(kAll, v, src),
+                                    __shfl_sync(kAll, inst, src), __shfl_sync(kAll, face, src)};
+                if (o == lane && closer_hit(w.best, c.t, c.inst, c.face)) {
+                    w.best = c;
+                    closer = true;
+                }
+            }
+            if (closer) w.tmax_box = prune_limit(w.best.t, w.world.o().x, w.world.d().x, S.scene_abs_x);
+        } else if (kMode == kTraceOcclusion) {
+            const float limit = __shfl_sync(kAll, w.tmax_box, static_cast<int>(own));
+            const uint32_t blocked = __reduce_or_sync(kAll, hit && t < limit ? 1u << own : 0u);
+            if ((blocked >> lane) & 1u) {
+                w.best.inst = 0u;  // (which instance it was is not asked for)
+                over = over || walking;
+                walking = false;
+            }
+        } else {
+            for (uint32_t m = __ballot_sync(kAll, hit); m != 0u; m &= m - 1u) {
+                const int src = __ffs(m) - 1;
+                const uint32_t o = __shfl_sync(kAll, own, src), ci = __shfl_sync(kAll, inst, src);
+                if (o == lane) {
+                    w.best.inst = ci;
+                    over = over || walking;
+                    walking = false;
+                }
+            }
+        }
+        const uint32_t rem = cnt > 32u ? cnt - 32u : 0u;
+        uint2 e = make_uint2(0u, 0u);
+        uint32_t o = 0;
+        if (lane < rem) {
+            e = Q.pair[32u + lane];
+            o = Q.owner[32u + lane];
+        }
+        __syncwarp();
+        if (lane < rem) {
+            Q.pair[lane] = e;
+            Q.owner[lane] = static_cast<uint8_t>(o);
+        }
+        if (lane == 0) Q.count = rem;
+        __syncwarp();
+    };
+
     for (;;) {
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !active);
+        const uint32_t idle = __ballot_sync(kAll, !walking && !over);
         if (!exhausted && idle != 0u) {
             const uint32_t cnt = __popc(idle);
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(cnt));
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            base = __shfl_sync(kAll, base, 0);
             if (base + cnt >= n) exhausted = true;
-            if (!active) {
+            if (!walking && !over) {
                 const unsigned long long q = base + __popc(idle & lt_mask);
                 if (q < n) {
                     item = q;
@@ -555,21 +658,35 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
                     float tm = tmax;
                     const uint32_t root = fetch(q, o, d, tm);
                     w.init(S, root, o, d, tm);
-                    stack.reset();
-                    active = true;
+                    walking = true;
                 }
             }
         }
-        if (__ballot_sync(0xFFFFFFFFu, active) == 0u) {
+        if (__ballot_sync(kAll, walking) == 0u) {  // (no walk is over with pairs left: the loop below drained them)
             if (exhausted) break;
             continue;
         }
-        while (active) {
-            if (w.step(S, stack, err, counts)) {
-                finish(item, w.best);
-                active = false;
+        for (;;) {
+            if (walking && w.step(S, stack, err, counts, leaves, group)) {
+                walking = false;
+                over = true;
             }
-            if (!exhausted && __popc(__ballot_sync(__activemask(), active)) < kRefillLanes) break;
+            __syncwarp();
+            const uint32_t walkers = __popc(__ballot_sync(kAll, walking));
+            // Once the list is exhausted there is nothing to refill: every few steps, which keeps a round's latency
+            // out of most steps of the last, longest walks (418 rays in host memory: 98 us a call before the queue,
+            // 103 with a round every step, 88 with one every 4; 8 the same).
+            const bool drain = !exhausted ? walkers < kRefillLanes : walkers == 0u || (++tail_steps % kTailSteps) == 0u;
+            for (;;) {
+                const uint32_t cnt = min(__shfl_sync(kAll, Q.count, 0), kQueueCap);
+                if (cnt < 32u && !(drain && cnt != 0u)) break;
+                round(cnt);
+            }
+            if (drain) {  // the queue is empty: every walk that is over has its result
+                if (over) finish(item, w.best);
+                over = false;
+                if (!exhausted || walkers == 0u) break;
+            }
         }
     }
 }
@@ -621,7 +738,7 @@ __device__ __forceinline__ bool make_frustum(const LevelRay (&r)[kRays], uint32_
 }
 
 // Bounds over the packet of one axis's slab terms: a = s * inv and o = (p - org) * inv, the two values
-// visit_node forms per ray (t = fma(q, a, o) for a plane byte q). Each is a product or difference of the
+// a ray's slab test is made of (t = fma(q, a, o) for a plane byte q). Each is a product or difference of the
 // lanes' values, so rounding to nearest keeps them within the products and differences of the extremes.
 __device__ __forceinline__ void axis_bounds(float p, float s, float omin, float omax, float imin, float imax,
                                             float &alo, float &ahi, float &olo, float &ohi) {
@@ -633,11 +750,11 @@ __device__ __forceinline__ void axis_bounds(float p, float s, float omin, float 
     ohi = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
 }
 
-// visit_node for a whole packet at once: each 8-lane group of the warp visits node `idx` (its own: the groups
+// The slab test for a whole packet at once: each 8-lane group of the warp visits node `idx` (its own: the groups
 // may visit different nodes), lane k testing child slot k mod 8 against the packet's bounds, and the group
 // ORs the results. fma(q, a, o) grows with a (q >= 0) and with o, so the lower bound of each near-plane t and
 // the upper bound of each far-plane t take the extremes of a and o: a child passes whenever it passes for at
-// least one lane's own ray with that lane's tmax (<= `tmax`), as visit_node computes it, and may pass for
+// least one lane's own ray with that lane's tmax (<= `tmax`), in that form, and may pass for
 // none (the packet then visits a node that none of its rays needs, which only costs time). Every lane of the
 // warp must call this; the result is the same in every lane of a group.
 __device__ __forceinline__ void visit_node_frustum(const uint4 *__restrict__ nodes, uint32_t idx,
@@ -686,7 +803,7 @@ __device__ __forceinline__ void visit_node_frustum(const uint4 *__restrict__ nod
 // leader's octant, every lane testing its own rays against each triangle. When all the packet's rays share
 // that octant (checked per level, TLAS and each BLAS), a node's 8 children are tested once for the whole
 // packet (visit_node_frustum: one child per lane against the bounds of all its rays); otherwise every lane
-// tests them with its own rays (visit_node) and takes only the children they hit. Either way a ray is tested
+// tests them with its own rays (visit_slots) and takes only the children they hit. Either way a ray is tested
 // against every box and triangle its own walk would reach, and pruned only beyond its own best t; it may be
 // tested against more. Its result is still the smallest world t over every triangle and sphere it hits
 // (exact ties to the smaller (instance, face)), which no visiting order or extra test changes: the results
@@ -767,7 +884,7 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                 wo[r] = o0;
                 wd[r] = d0;
             }
-            setup_level(ray[r], wo[r], wd[r]);
+            setup_level<true>(ray[r], wo[r], wd[r]);
             best[r] = TraceResult{kFltMax, 0.f, 0.f, kInvalid, kInvalid};
             tmax_box[r] = kFltMax;
 #if SPK_PACKET_WORLD_SMEM
@@ -863,12 +980,11 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                 uint32_t hits = 0u;
 #pragma unroll
                 for (int r = 0; r < kRays; ++r) {
-                    uint2 ng, tg;
-                    visit_node(S.nodes, node_idx, ray[r], order, mine ? tmax_box[r] : -1.f, ng, tg);
-                    hits |= (ng.y & 0xFF000000u) | tg.y;
-                    ngroup.x = ng.x;
-                    tgroup.x = tg.x;
-                    ngroup.y = (ngroup.y & ~0xFFu) | (ng.y & 0xFFu);  // the child's imask
+                    const NodeHits h = visit_slots(S.nodes, node_idx, ray[r], mine ? tmax_box[r] : -1.f);
+                    hits |= (order_slots(h.hit & h.imask, order) << 24) | leaf_items(h.hit & ~h.imask, h.meta);
+                    ngroup.x = h.child_base;
+                    tgroup.x = h.item_base;
+                    ngroup.y = (ngroup.y & ~0xFFu) | h.imask;  // the child's imask
                 }
                 nown = hits & 0xFF000000u;
                 town = hits & 0x00FFFFFFu;
@@ -902,7 +1018,7 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                         const float wt = world_t(S.instances[cur_inst], ray[r], t, ro, rd);
                         if (wt > 0.f && closer_hit(best[r], wt, cur_inst, face)) {
                             best[r] = TraceResult{wt, u, v, cur_inst, face};
-                            tmax_box[r] = prune_limit(wt, ro, rd, S.scene_abs_x);
+                            tmax_box[r] = prune_limit(wt, ro.x, rd.x, S.scene_abs_x);
                         }
                     }
                 } else {
@@ -917,7 +1033,7 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                             if (sphere_hit(I, ray[r].o, ray[r].d, t) && t > 0.f &&
                                 closer_hit(best[r], t, inst, kInvalid)) {
                                 best[r] = TraceResult{t, 0.f, 0.f, inst, kInvalid};
-                                tmax_box[r] = prune_limit(t, ray[r].o, ray[r].d, S.scene_abs_x);
+                                tmax_box[r] = prune_limit(t, ray[r].o.x, ray[r].d.x, S.scene_abs_x);
                             }
                         }
                     } else if (I.blas_root != kInvalid) {
@@ -930,7 +1046,7 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                         cur_inst = inst;
 #pragma unroll
                         for (int r = 0; r < kRays; ++r)
-                            setup_level(ray[r], xform_point(I.minv, ray[r].o), xform_dir(I.minv, ray[r].d));
+                            setup_level<true>(ray[r], xform_point(I.minv, ray[r].o), xform_dir(I.minv, ray[r].d));
                         const uint32_t entering = __ballot_sync(kAll, mine);  // not empty: the group had bit k
                         order = __shfl_sync(kAll, ray[0].oct, __ffs(entering) - 1);
                         packed = make_frustum(ray, order, frustum);
@@ -947,9 +1063,9 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
 #pragma unroll
                     for (int r = 0; r < kRays; ++r) {
 #if SPK_PACKET_WORLD_SMEM
-                        setup_level(ray[r], world_o(r), world_d(r));
+                        setup_level<true>(ray[r], world_o(r), world_d(r));
 #else
-                        setup_level(ray[r], wo[r], wd[r]);
+                        setup_level<true>(ray[r], wo[r], wd[r]);
 #endif
                     }
                     order = top_order;

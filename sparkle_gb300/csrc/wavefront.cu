@@ -250,29 +250,27 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
     const unsigned long long first = kPackets == 2 ? 0ull : kPackets == 1 ? p2 : p1;
     const unsigned long long n = (kPackets == 2 ? p2 : kPackets == 1 ? p1 : len) - first;
     if (n == 0) return;
-    uint32_t err = 0, done = 0;
+    uint32_t err = 0;
     TraceCounts tc;
     const uint32_t *queue = s.queue[in_queue] + first;
-    uint32_t pid = 0;
     auto fetch = [&](unsigned long long q, f3 &o, f3 &d, float &) {
-        pid = queue[q];
+        const uint32_t pid = queue[q];
         load_ray(s, pid, o, d);
         return kBatch ? s.slot_root[pid] : S.tlas_root;
     };
-    auto store = [&](uint32_t p, const TraceResult &h) {
-        s.hit[p] = make_float4(h.t, h.u, h.v, __uint_as_float(h.inst));
-        s.hit_face[p] = h.face;
-        ++done;
+    auto finish = [&](unsigned long long q, const TraceResult &h) {
+        const uint32_t pid = queue[q];
+        s.hit[pid] = make_float4(h.t, h.u, h.v, __uint_as_float(h.inst));
+        s.hit_face[pid] = h.face;
     };
     if constexpr (kPackets != 0) {
         walk_packets<kCount, kPackets>(S, &counters->queue_counters[kPackets == 2 ? kPacket2Cursor : kPacketCursor], n,
-                                       err, &tc, fetch,
-                                       [&](unsigned long long q, const TraceResult &h) { store(queue[q], h); });
+                                       err, &tc, fetch, finish);
     } else {
         walk_persistent<kTraceClosest, kCount>(S, &counters->queue_counters[kCursor], n, kFltMax, err, &tc, fetch,
-                                               [&](unsigned long long, const TraceResult &h) { store(pid, h); });
+                                               finish);
     }
-    warp_add_u64(&counters->extension_rays, done);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&counters->extension_rays, n);
     if (kCount) {
         warp_add_u64(&counters->node_visits, tc.nodes);
         warp_add_u64(&counters->tri_tests, tc.tris);
@@ -755,19 +753,18 @@ __global__ void __launch_bounds__(128, SPK_SHADOW_MIN_BLOCKS) k_wf_shadow(DevSce
                                                                        Counters *counters) {
     uint32_t err = 0;
     const unsigned long long n = counters->queue_counters[kShadowLen];
-    uint32_t e = 0;
     walk_persistent<kTraceOcclusion, false>(
         S, &counters->queue_counters[kShadowCursor], n, kFltMax, err, nullptr,
         [&](unsigned long long q, f3 &o, f3 &d, float &tmax) {
-            e = s.shadow_queue[q];
+            const uint32_t e = s.shadow_queue[q];
             const float4 o4 = s.shadow_o[e], d4 = s.shadow_d[e];
             o = mk3(o4.x, o4.y, o4.z);
             d = mk3(d4.x, d4.y, d4.z);
             tmax = o4.w;
             return kBatch ? s.slot_root[e >> 1] : S.tlas_root;
         },
-        [&](unsigned long long, const TraceResult &h) {
-            if (h.inst == kInvalid) reinterpret_cast<float *>(s.nee_contrib + e)[3] = 2.f;
+        [&](unsigned long long q, const TraceResult &h) {
+            if (h.inst == kInvalid) reinterpret_cast<float *>(s.nee_contrib + s.shadow_queue[q])[3] = 2.f;
         });
     if (err) atomicOr(&counters->error_flags, err);
 }

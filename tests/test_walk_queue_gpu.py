@@ -1,0 +1,56 @@
+"""The persistent walk's triangle queue where it runs full: every ray of a warp reaches leaf after leaf of stacked
+triangles, up to 24 per node and lane against room for 64 per warp, so that most go back to the ray's stack and are
+queued again. Hits must equal the oracle's, at ray counts around a warp's 32 lanes."""
+import numpy as np
+import pytest
+
+import oracle
+from sparkle_gb300 import abi, native, scenes
+
+from parity import INVALID, classify_hits, oracle_hits
+
+pytestmark = pytest.mark.gpu
+
+
+def stacked_triangles(layers: int):
+    """`layers` large triangles, one above the other and slightly tilted, as two instances (one turned and scaled),
+    with an analytic sphere between them."""
+    rng = np.random.default_rng(layers)
+    z = np.linspace(0.0, 1.0, layers)
+    base = np.array([[-4.0, -3.0], [4.0, -3.0], [0.0, 5.0]])
+    pos = np.zeros((layers, 3, 3))
+    pos[:, :, :2] = base
+    pos[:, :, 2] = z[:, None] + rng.uniform(-0.3, 0.3, (layers, 3)) / layers
+    pos = pos.reshape(-1, 3)
+    nrm = np.tile([0.0, 0.0, 1.0], (len(pos), 1))
+    mesh = abi.Mesh(pos, nrm, np.arange(len(pos)).reshape(-1, 3))
+    mats = [abi.Material.lambertian((0.5, 0.5, 0.5))]
+    lin = scenes._rot_z(0.4) @ np.diag([1.2, 0.9, 1.1])
+    inst = [abi.Instance(0, 0), abi.Instance(0, 0, scenes._affine(lin, (0.2, -0.1, -3.0))),
+            abi.Instance(0, 0, scenes._affine(np.eye(3), (0.5, 0.5, -1.0)), sphere=True, radius=0.8)]
+    return abi.Scene([mesh], inst, mats, abi.Sky(), name=f"stack{layers}")
+
+
+@pytest.mark.parametrize("layers", [1, 24, 200])
+@pytest.mark.parametrize("count", [1, 31, 32, 33, 4097])
+def test_stacked_triangles_match_the_oracle(layers, count):
+    scene = stacked_triangles(layers)
+    rng = np.random.default_rng(count)
+    target = np.stack([rng.uniform(-3, 3, count), rng.uniform(-2, 3, count), rng.uniform(-3, 1, count)], 1)
+    origin = np.stack([rng.uniform(-3, 3, count), rng.uniform(-3, 3, count), np.where(rng.random(count) < 0.5, 6.0, -8.0)], 1)
+    d = target - origin
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = abi.rays_to_array(origin, d)
+    ref_scene = oracle.OracleScene(scene)
+    ctx = native.Context(0)
+    ctx.set_scene(scene)
+    got = ctx.trace(rays)
+    assert ctx.stats()["error_flags"] == 0
+    assert ctx.stats()["extension_rays"] == count
+    ref, _ = oracle_hits(ref_scene, rays, oracle.PRUNED)
+    c = classify_hits(got, ref)
+    assert c["exact"] + c["tie"] == count, c
+    any_hit = ctx.trace(rays, any_hit=True)
+    sphere = ref["face"][ref["prim"] != INVALID] == INVALID  # (an any-hit query takes a sphere behind the ray too)
+    assert not ((any_hit["prim"] == INVALID) & (ref["prim"] != INVALID)).any(), sphere.sum()
+    ctx.close()
