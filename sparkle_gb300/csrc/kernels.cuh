@@ -32,6 +32,7 @@ struct Counters {
     unsigned long long node_visits;
     unsigned long long tri_tests;
     unsigned long long queue_counters[12];
+    unsigned int seed_base, seed_step;  // multi-frame pass: frame k's samples are seeded with seed_base + k * seed_step
 };
 
 // Sum of a per-thread count over the active lanes of a warp, added once per warp.
@@ -49,6 +50,8 @@ struct LaunchEvents {
     int used = 0;
     float graph_ms = 0.f;   // traversal time measured inside replayed CUDA graphs
     int graph_launches = 0;  // traversal launches inside replayed CUDA graphs
+    cudaEvent_t *graph_pairs = nullptr;  // events of a replay whose times are still to be read (after the stream is done)
+    int graph_pending = 0;
     // cudaEventRecordExternal while a stream is captured: the record becomes a graph node that every replay
     // performs (a plain record under capture only orders work inside the graph).
     unsigned record_flags = cudaEventRecordDefault;

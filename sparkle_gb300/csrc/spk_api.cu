@@ -189,8 +189,6 @@ struct spk_ctx {
     // The frame buffer that bookkeeping belongs to: nullptr = fb; otherwise the caller's buffer that
     // spk_render_noalloc accumulated into last. Rendering into another buffer restarts the accumulation.
     const void *accum_target = nullptr;
-    std::vector<float> frame_weights;    // multi-frame wavefront: per-frame moving-average weight
-    std::vector<uint32_t> frame_seeds;   // multi-frame wavefront: per-frame seed base
 
     // counters
     Counters *counters = nullptr;  // device
@@ -344,6 +342,7 @@ cudaError_t prepare_events(spk_ctx *ctx, size_t pairs) {
     ctx->launch_events.used = 0;
     ctx->launch_events.graph_ms = 0.f;
     ctx->launch_events.graph_launches = 0;
+    ctx->launch_events.graph_pending = 0;
     return cudaSuccess;
 }
 
@@ -1386,33 +1385,25 @@ static spk_status render_impl(spk_ctx *ctx, uint32_t num_frames) {
         return cuda_fail(ctx, e, "counter reset");
     if ((e = cudaEventRecord(ctx->ev_start, ctx->stream)) != cudaSuccess) return cuda_fail(ctx, e, "event");
     if (wavefront && ctx->tuning.multi_frame && num_frames > 0) {
-        // All frames in one regenerating wavefront: run the per-frame bookkeeping ahead on the host and hand
-        // the kernels each frame's weight and seed base (the spatial fill, when on, runs per frame in the
+        // All frames in one regenerating wavefront: the per-frame bookkeeping runs ahead on the host, the kernels derive
+        // each frame's weight and seed base from its start (the spatial fill, when on, runs per frame in the
         // resolve over that frame's samples and first-hit normals).
-        ctx->frame_weights.resize(num_frames);
-        ctx->frame_seeds.resize(num_frames);
-        bool clear = false;
+        FrameSchedule sched{0u, ctx->spp_eff, 0u, ctx->cfg.max_spp, ctx->dirty};
         for (uint32_t f = 0; f < num_frames; ++f) {
             if (ctx->dirty) {
                 ctx->cumulated = 0;
                 ctx->pending = 0;
+                ctx->dispatched = ctx->cfg.sample_offset;
+                ctx->dirty = false;
             }
             ctx->cumulated = std::min(ctx->cfg.max_spp, ctx->cumulated + ctx->pending);
-            ctx->pending = 0;
-            if (ctx->dirty) {
-                clear = true;
-                ctx->dirty = false;
-                ctx->dispatched = ctx->cfg.sample_offset;
+            if (f == 0) {
+                sched.seed_base = ctx->dispatched;
+                sched.cumulated = ctx->cumulated;
             }
-            ctx->frame_seeds[f] = ctx->dispatched;
-            ctx->frame_weights[f] =
-                static_cast<float>(ctx->cumulated) / static_cast<float>(ctx->cumulated + ctx->spp_eff);
             ctx->dispatched += ctx->spp_eff;
-            ctx->pending += ctx->spp_eff;
+            ctx->pending = ctx->spp_eff;
         }
-        if (clear &&
-            (e = cudaMemsetAsync(ctx->fb.ptr, 0, ctx->fb.count * sizeof(float4), ctx->stream)) != cudaSuccess)
-            return cuda_fail(ctx, e, "frame buffer clear");
         RenderParams p{0u, ctx->cfg.bounce, ctx->cfg.rng, ctx->cfg.seed, ctx->cfg.spatial_denoise, ctx->cfg.enable_nee};
         uint32_t launches = 0;
         ctx->chunk_graph.enabled = ctx->tuning.cuda_graph != 0;
@@ -1422,12 +1413,15 @@ static spk_status render_impl(spk_ctx *ctx, uint32_t num_frames) {
         const uint64_t npix = static_cast<uint64_t>(ctx->cfg.width) * ctx->cfg.height;
         const uint64_t per_pixel = std::min<uint64_t>({ctx->tuning.path_slots_per_pixel, num_frames, kFramesPerPass});
         const uint64_t slots = std::max<uint64_t>(npix, std::min<uint64_t>(npix * per_pixel, kMaxPathSlots));
-        if (ctx->wf.capacity < slots && (e = wavefront_alloc(ctx->wf, static_cast<uint32_t>(slots))) != cudaSuccess)
+        if (ctx->wf.capacity < slots && (e = wavefront_alloc(ctx->wf, static_cast<uint32_t>(slots))) != cudaSuccess) {
+            ctx->dirty = ctx->dirty || sched.clear;  // the resolve that would have cleared the buffer does not run
             return cuda_fail(ctx, e, "path state allocation");
-        e = launch_render_multiframe(ctx->scene, ctx->cam, fbuf, p, num_frames, ctx->frame_weights.data(),
-                                     ctx->frame_seeds.data(), count, ctx->counters, ctx->wf, ctx->num_sms,
-                                     ctx->stream, &launches, &ctx->launch_events, wf_tuning(ctx), &ctx->chunk_graph);
+        }
+        e = launch_render_multiframe(ctx->scene, ctx->cam, fbuf, p, num_frames, sched, count, ctx->counters, ctx->wf,
+                                     ctx->num_sms, ctx->stream, &launches, &ctx->launch_events, wf_tuning(ctx),
+                                     &ctx->chunk_graph);
         if (e != cudaSuccess) {
+            ctx->dirty = ctx->dirty || sched.clear;
             const std::string what = std::string("multi-frame wavefront (") + wavefront_error_site() + ")";
             return cuda_fail(ctx, e, what.c_str());
         }
@@ -1954,7 +1948,13 @@ spk_status spk_get_stats(spk_ctx *ctx, spk_stats *out) {
         cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop);
         ctx->last.device_ms = ms;
         float tms = 0.f;
-        const LaunchEvents &le = ctx->launch_events;
+        LaunchEvents &le = ctx->launch_events;
+        for (int k = 0; k < le.graph_pending; ++k) {
+            float x = 0.f;
+            cudaEventElapsedTime(&x, le.graph_pairs[2 * k], le.graph_pairs[2 * k + 1]);
+            le.graph_ms += x;
+        }
+        le.graph_pending = 0;
         for (int k = 0; k < le.used; ++k) {
             float x = 0.f;
             cudaEventElapsedTime(&x, le.pairs[2 * k], le.pairs[2 * k + 1]);

@@ -244,6 +244,14 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
                                        : kPackets == 1 ? SPK_PACKET_MIN_BLOCKS
                                                        : SPK_WALK_MIN_BLOCKS)
     k_wf_extend(DevScene S, WavefrontState s, int in_queue, Counters *counters) {
+    // The stage's own resets, in place of memset nodes between the kernels: the queues the shade stage fills (nothing
+    // reads them now). The shade stage zeroes the walks' cursors in turn.
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        counters->queue_counters[in_queue ^ 1] = 0u;
+        counters->queue_counters[kShadowLen] = 0u;
+        counters->queue_counters[kNeeLen] = 0u;
+        counters->queue_counters[kShadowCursor] = 0u;
+    }
     const unsigned long long len = counters->queue_counters[in_queue];
     const unsigned long long p1 = min(counters->queue_counters[kPacketQueue], len);
     const unsigned long long p2 = min(counters->queue_counters[kPacket2Queue], p1);
@@ -278,16 +286,24 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
     if (err) atomicOr(&counters->error_flags, err);
 }
 
+// After an extend stage: its cursors back to zero, and no packet prefix (the next queue is mixed).
+__device__ __forceinline__ void reset_walk(Counters *counters) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        counters->queue_counters[kCursor] = 0u;
+        counters->queue_counters[kPacketCursor] = 0u;
+        counters->queue_counters[kPacket2Cursor] = 0u;
+        counters->queue_counters[kPacketQueue] = 0u;
+        counters->queue_counters[kPacket2Queue] = 0u;
+    }
+}
+
 template <int kKind, int kNee>
 __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_wf_shade(DevScene S, FrameBuffers fb, RenderParams p, WavefrontState s,
                                                   int in_queue, uint32_t bounce, Counters *counters) {
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the next queue is mixed
-        counters->queue_counters[kPacketQueue] = 0u;
-        counters->queue_counters[kPacket2Queue] = 0u;
-    }
+    reset_walk(counters);
     const uint32_t *queue = s.queue[in_queue];
     for (unsigned long long q0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x; q0 < n;
          q0 += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
@@ -349,7 +365,8 @@ __device__ __forceinline__ uint32_t item_pixel(uint32_t q, uint32_t w, uint32_t 
 template <int kKind>
 __device__ __forceinline__ void start_item(const DevCamera &cam, const RenderParams &p, const WavefrontState &s,
                                            uint32_t slot, uint32_t item, uint32_t w, uint32_t h,
-                                           uint32_t frame_base, uint32_t total_items) {
+                                           uint32_t frame_base, uint32_t total_items, uint32_t seed_base,
+                                           uint32_t seed_step) {
     const uint32_t npix = w * h;
 #if SPK_ITEM_ORDER == 1
     const uint32_t frames = total_items / npix;
@@ -358,7 +375,7 @@ __device__ __forceinline__ void start_item(const DevCamera &cam, const RenderPar
     (void)total_items;
     const uint32_t k = item / npix, pid = item_pixel(item - k * npix, w, h);
 #endif
-    start_path<kKind>(cam, p, s, slot, pid % w, pid / w, w, h, s.frame_seed[frame_base + k]);
+    start_path<kKind>(cam, p, s, slot, pid % w, pid / w, w, h, seed_base + (frame_base + k) * seed_step);
     s.slot_item[slot] = k * npix + pid;
     s.slot_state[slot] = 0u;
     if (p.spatial_denoise) s.sample_normals[k * npix + pid] = make_float4(0.f, 0.f, 0.f, 0.f);  // a miss: sky
@@ -368,14 +385,17 @@ __device__ __forceinline__ void start_item(const DevCamera &cam, const RenderPar
 template <int kKind>
 __global__ void __launch_bounds__(128) k_mf_generate(DevCamera cam, FrameBuffers fb, RenderParams p,
                                                      WavefrontState s, uint32_t frame_base, uint32_t initial,
-                                                     uint32_t total_items, uint32_t packets, Counters *counters) {
+                                                     uint32_t total_items, uint32_t packets, uint32_t seed_base,
+                                                     uint32_t seed_step, Counters *counters) {
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= initial) return;
-    start_item<kKind>(cam, p, s, slot, slot, fb.width, fb.height, frame_base, total_items);
+    start_item<kKind>(cam, p, s, slot, slot, fb.width, fb.height, frame_base, total_items, seed_base, seed_step);
     s.queue[0][slot] = slot;
     if (slot == 0) {
         counters->queue_counters[kLen0] = initial;
         counters->queue_counters[kNextItem] = initial;
+        counters->seed_base = seed_base;
+        counters->seed_step = seed_step;
         const uint32_t frames = total_items / (fb.width * fb.height);
         const bool pk = SPK_ITEM_ORDER == 1 && packets && frames >= kPacketMinSamples;
         counters->queue_counters[kPacketQueue] = pk ? initial : 0u;
@@ -392,10 +412,7 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_mf_shade(DevScene
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the next queue is mixed
-        counters->queue_counters[kPacketQueue] = 0u;
-        counters->queue_counters[kPacket2Queue] = 0u;
-    }
+    reset_walk(counters);
     const uint32_t *queue = s.queue[in_queue];
     const uint32_t lane = threadIdx.x & 31u;
     for (unsigned long long q0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x; q0 < n;
@@ -433,7 +450,7 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_mf_shade(DevScene
                 const unsigned long long item = base + __popc(need_mask & ((1u << lane) - 1u));
                 if (item < total_items) {
                     start_item<kKind>(cam, p, s, slot, static_cast<uint32_t>(item), fb.width, fb.height, frame_base,
-                                      total_items);
+                                      total_items, counters->seed_base, counters->seed_step);
                     push = true;
                 }
             }
@@ -604,18 +621,22 @@ __device__ __forceinline__ float aces_tonemap(float c, float exposure) {
 
 // DenoisePass temporal lerp of every sample of the pass, in frame order per pixel
 // (fb = new + (fb - new) * w_k, CPURenderer.cpp:534-543), then ToneMappingPass (:554-576).
-__global__ void __launch_bounds__(256) k_mf_resolve(FrameBuffers fb, WavefrontState s, uint32_t frame_base,
-                                                    uint32_t frames, float exposure, uint32_t spatial) {
+__global__ void __launch_bounds__(256) k_mf_resolve(FrameBuffers fb, WavefrontState s, FrameSchedule sched,
+                                                    uint32_t frame_base, uint32_t frames, float exposure,
+                                                    uint32_t spatial) {
     const uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t npix = fb.width * fb.height;
     if (pid >= npix) return;
-    float4 a = fb.fb[pid];
+    float4 a = sched.clear && frame_base == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : fb.fb[pid];
     for (uint32_t k = 0; k < frames; ++k) {
         float4 n = s.samples[static_cast<size_t>(k) * npix + pid];
         if (spatial)  // DenoisePass's spatial fill of frame k's G-buffer (CPURenderer.cpp:452-526)
             n = spatial_fill(s.samples + static_cast<size_t>(k) * npix, s.sample_normals + static_cast<size_t>(k) * npix,
                              pid % fb.width, pid / fb.width, fb.width, fb.height, n);
-        const float f = s.frame_weight[frame_base + k];
+        const uint32_t c = static_cast<uint32_t>(
+            min(static_cast<unsigned long long>(sched.max_spp),
+                sched.cumulated + static_cast<unsigned long long>(frame_base + k) * sched.spp));
+        const float f = static_cast<float>(c) / static_cast<float>(c + sched.spp);
         a = make_float4(n.x + (a.x - n.x) * f, n.y + (a.y - n.y) * f, n.z + (a.z - n.z) * f, n.w + (a.w - n.w) * f);
     }
     fb.fb[pid] = a;
@@ -696,10 +717,7 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_b_shade(DevScene 
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the next queue is mixed
-        counters->queue_counters[kPacketQueue] = 0u;
-        counters->queue_counters[kPacket2Queue] = 0u;
-    }
+    reset_walk(counters);
     const uint32_t *queue = s.queue[in_queue];
     const uint32_t lane = threadIdx.x & 31u;
     for (unsigned long long q0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x; q0 < n;
@@ -814,7 +832,7 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_nee_accumulate(De
                     const unsigned long long item = base + __popc(need_mask & ((1u << lane) - 1u));
                     if (kMode == 1 && item < total_items) {
                         start_item<kKind>(cam, p, s, slot, static_cast<uint32_t>(item), fb.width, fb.height,
-                                          frame_base, total_items);
+                                          frame_base, total_items, counters->seed_base, counters->seed_step);
                         push = true;
                     } else if (kMode == 2 && item < b.item_hi) {
                         start_item_batch<kKind>(S, b, s, slot, item);
@@ -904,10 +922,6 @@ uint32_t pass_packet_forms(uint32_t frames, const WfTuning &tuning) {
 
 cudaError_t launch_extend(const DevScene &scene, const WavefrontState &s, int in, bool count, Counters *counters,
                           unsigned grid, cudaStream_t stream, LaunchEvents *ev, bool batch, uint32_t packet_forms) {
-    unsigned long long *qc = counters->queue_counters;
-    static_assert(kPacketCursor == kCursor + 1 && kPacket2Cursor == kCursor + 2, "one reset for the cursors");
-    cudaError_t e = cudaMemsetAsync(qc + kCursor, 0, 3 * sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
     if (ev) ev->before(stream);
     if (batch) {
         if (packet_forms & 2u)
@@ -966,11 +980,6 @@ void enqueue_shadow_stage(const DevScene &scene, const DevCamera &cam, const Fra
     acc<<<shade_grid, 128, 0, stream>>>(cam, fbuf, p, scene, b, s, out_queue, frame_base, total_items, counters);
 }
 
-// Resets the shadow stage's counters (queued rays, vertices, walk cursor) before a shade stage.
-cudaError_t reset_shadow_counters(Counters *counters, cudaStream_t stream) {
-    return cudaMemsetAsync(counters->queue_counters + kShadowLen, 0, 3 * sizeof(unsigned long long), stream);
-}
-
 }  // namespace
 
 cudaError_t wavefront_alloc_nee(WavefrontState &s) {
@@ -1023,7 +1032,7 @@ cudaError_t wavefront_alloc(WavefrontState &s, uint32_t capacity) {
 void wavefront_free(WavefrontState &s) {
     void *ptrs[] = {s.ray_a,      s.ray_b,     s.thr,     s.color,        s.rng,        s.hit,
                     s.hit_face,   s.queue[0],  s.queue[1], s.sort_keys,   s.slot_state, s.slot_item,
-                    s.samples,    s.frame_weight, s.frame_seed, s.prev_pdf, s.sort_hist, s.slot_req,
+                    s.samples,    s.prev_pdf, s.sort_hist, s.slot_req,
                     s.slot_root,  s.sort_keys2, s.shadow_o, s.shadow_d, s.nee_contrib, s.shadow_queue,
                     s.nee_list,   s.sample_normals};
     for (void *p : ptrs)
@@ -1066,7 +1075,6 @@ cudaError_t launch_render_wavefront(const DevScene &scene, const DevCamera &cam,
     const unsigned shadow_grid = shadow_blocks(num_sms, tuning.extend_blocks_per_sm);
     for (uint32_t b = 0; b < p.bounce; ++b) {
         const int in = static_cast<int>(b & 1u), out = in ^ 1;
-        if ((e = cudaMemsetAsync(qc + out, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
         WavefrontState se = s;
         if (tuning.ray_sort) {
             se = enqueue_ray_sort(scene, s, in, counters, num_sms, stream);
@@ -1080,7 +1088,6 @@ cudaError_t launch_render_wavefront(const DevScene &scene, const DevCamera &cam,
             ss = enqueue_material_sort(scene, se, in, counters, num_sms, stream);
             nl += 3;
         }
-        if (nee == kNeeDeferred && (e = reset_shadow_counters(counters, stream)) != cudaSuccess) return e;
         pick_wf_shade(p.rng, nee)<<<shade_blocks, 128, 0, stream>>>(scene, fbuf, p, ss, in, b, counters);
         ++nl;
         if (nee == kNeeDeferred) {
@@ -1102,8 +1109,8 @@ thread_local const char *t_site = "";
 const char *wavefront_error_site() { return t_site; }
 
 cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam, const FrameBuffers &fbuf,
-                                     const RenderParams &p, uint32_t num_frames, const float *weights,
-                                     const uint32_t *seeds, bool count, Counters *counters, WavefrontState &s,
+                                     const RenderParams &p, uint32_t num_frames, const FrameSchedule &frames_of,
+                                     bool count, Counters *counters, WavefrontState &s,
                                      int num_sms, cudaStream_t stream, uint32_t *launches, LaunchEvents *ev,
                                      const WfTuning &tuning, ChunkGraph *graph) {
     uint32_t nl = 0;
@@ -1114,16 +1121,6 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
     cudaError_t e;
     const int nee = nee_mode(p.enable_nee, tuning);
     if (nee == kNeeDeferred && (e = wavefront_alloc_nee(s)) != cudaSuccess) return e;
-    if (s.frame_capacity < num_frames) {
-        if (s.frame_weight) cudaFree(s.frame_weight);
-        if (s.frame_seed) cudaFree(s.frame_seed);
-        s.frame_weight = nullptr;
-        s.frame_seed = nullptr;
-        s.frame_capacity = 0;
-        if ((e = dmalloc(s.frame_weight, num_frames)) != cudaSuccess) return e;
-        if ((e = dmalloc(s.frame_seed, num_frames)) != cudaSuccess) return e;
-        s.frame_capacity = num_frames;
-    }
     const uint32_t pass_frames = std::min(num_frames, kFramesPerPass);
     const size_t need = static_cast<size_t>(pass_frames) * npix;
     if (s.sample_capacity < need) {
@@ -1140,17 +1137,12 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
         if ((e = dmalloc(s.sample_normals, need)) != cudaSuccess) return e;
         s.normal_capacity = need;
     }
-    if ((e = cudaMemcpyAsync(s.frame_weight, weights, num_frames * sizeof(float), cudaMemcpyHostToDevice, stream)) !=
-            cudaSuccess ||
-        (e = cudaMemcpyAsync(s.frame_seed, seeds, num_frames * sizeof(uint32_t), cudaMemcpyHostToDevice, stream)) !=
-            cudaSuccess)
-        return e;
     unsigned long long *qc = counters->queue_counters;
     const unsigned shade_blocks = static_cast<unsigned>(num_sms) * tuning.shade_blocks_per_sm;
     const unsigned extend_grid = extend_blocks(num_sms, tuning.extend_blocks_per_sm);
     const unsigned shadow_grid = shadow_blocks(num_sms, tuning.extend_blocks_per_sm);
     constexpr uint32_t kChunk = kChunkIterations;
-    static_assert(kChunk % 2 == 0, "a chunk must keep the queue parity, so one graph serves every chunk");
+    static_assert(kChunk % 2 == 0, "a full chunk must keep the queue parity, so one graph serves every chunk");
     for (uint32_t f0 = 0; f0 < num_frames; f0 += kFramesPerPass) {
         const uint32_t frames = std::min(kFramesPerPass, num_frames - f0);
         const uint32_t packet_forms = pass_packet_forms(frames, tuning);
@@ -1159,21 +1151,20 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
         const uint64_t want = static_cast<uint64_t>(npix) * std::max(1u, tuning.slots_per_pixel);
         const uint32_t initial = static_cast<uint32_t>(
             std::min<uint64_t>({want, static_cast<uint64_t>(s.capacity), static_cast<uint64_t>(total_items)}));
-        if ((e = cudaMemsetAsync(qc, 0, sizeof(counters->queue_counters), stream)) != cudaSuccess) return e;
-        if (p.rng == 0) {
-            k_mf_generate<0><<<(initial + 127) / 128, 128, 0, stream>>>(cam, fbuf, p, s, f0, initial, total_items,
-                                                                     tuning.packets, counters);
-        } else {
-            k_mf_generate<1><<<(initial + 127) / 128, 128, 0, stream>>>(cam, fbuf, p, s, f0, initial, total_items,
-                                                                     tuning.packets, counters);
-        }
+        if (f0 != 0 && (e = cudaMemsetAsync(qc, 0, sizeof(counters->queue_counters), stream)) != cudaSuccess) return e;
+        auto *generate = p.rng == 0 ? k_mf_generate<0> : k_mf_generate<1>;
+        generate<<<(initial + 127) / 128, 128, 0, stream>>>(cam, fbuf, p, s, f0, initial, total_items, tuning.packets,
+                                                            frames_of.seed_base, frames_of.spp, counters);
+        // When every sample starts at once no slot starts a second one, so the paths take exactly `bounce` iterations:
+        // no more are launched than that, and the queue length need not be read back to know that they are over.
+        const bool at_once = initial == total_items;
+        const uint32_t iters = at_once ? std::min(p.bounce, kChunk) : kChunk;
         ++nl;
-        // One chunk: kChunk iterations of (reset the output queue, extend, shade).
+        // One chunk: `iters` iterations of (extend, shade).
         auto enqueue_chunk = [&](LaunchEvents *chunk_ev) -> cudaError_t {
             cudaError_t ce;
-            for (uint32_t c = 0; c < kChunk; ++c) {
+            for (uint32_t c = 0; c < iters; ++c) {
                 const int in = static_cast<int>(c & 1u), out = in ^ 1;
-                if ((ce = cudaMemsetAsync(qc + out, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return ce;
                 const WavefrontState se =
                     tuning.ray_sort ? enqueue_ray_sort(scene, s, in, counters, num_sms, stream) : s;
                 if ((ce = launch_extend(scene, se, in, count, counters, extend_grid, stream, chunk_ev, false,
@@ -1181,7 +1172,6 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                     return ce;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                if (nee == kNeeDeferred && (ce = reset_shadow_counters(counters, stream)) != cudaSuccess) return ce;
                 pick_mf_shade(p.rng, nee)<<<shade_blocks, 128, 0, stream>>>(scene, cam, fbuf, p, ss, in, f0,
                                                                             total_items, counters);
                 if (nee == kNeeDeferred)
@@ -1204,7 +1194,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                 uint32_t f0, total_items, count, num_sms;
                 Counters *counters;
                 cudaStream_t stream;
-                unsigned extend_grid, shade_grid, material_sort, ray_sort, nee_mode, packet_forms;
+                unsigned extend_grid, shade_grid, material_sort, ray_sort, nee_mode, packet_forms, iters;
             } key;
             std::memset(static_cast<void *>(&key), 0, sizeof(key));  // padding too: the key is compared bytewise
             key.scene = scene;
@@ -1224,6 +1214,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
             key.ray_sort = tuning.ray_sort;
             key.nee_mode = static_cast<unsigned>(nee);
             key.packet_forms = packet_forms;
+            key.iters = iters;
             const auto *kb = reinterpret_cast<const unsigned char *>(&key);
             graph_ev.pairs = graph->events;
             graph_ev.capacity = static_cast<int>(kChunk);
@@ -1281,29 +1272,39 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
             } else if ((e = enqueue_chunk(ev)) != cudaSuccess) {
                 return e;
             }
-            iter += kChunk;
+            iter += iters;
             nl += (2u + (tuning.material_sort ? 3u : 0u) + (tuning.ray_sort ? 3u : 0u) +
-                   (nee == kNeeDeferred ? 2u : 0u)) * kChunk +
+                   (nee == kNeeDeferred ? 2u : 0u)) * iters +
                   extend_launches(packet_forms) - 1u;
+            const bool over = at_once && iter >= p.bounce;
+            if (over && iter == iters && num_frames <= kFramesPerPass) {
+                if (use_graph && ev) {
+                    ev->graph_pairs = graph->events;
+                    ev->graph_pending = static_cast<int>(iters);
+                    ev->graph_launches = static_cast<int>(iters);
+                }
+                break;
+            }
             if ((e = cudaMemcpyAsync(s.host_len, qc, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream)) !=
                 cudaSuccess)
                 return e;
             if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
             t_site = "graph timing events";
             if (use_graph && ev) {
-                for (uint32_t c = 0; c < kChunk; ++c) {
+                for (uint32_t c = 0; c < iters; ++c) {
                     float x = 0.f;
                     if ((e = cudaEventElapsedTime(&x, graph->events[2 * c], graph->events[2 * c + 1])) != cudaSuccess)
                         return e;
                     ev->graph_ms += x;
                 }
-                ev->graph_launches += static_cast<int>(kChunk);
+                ev->graph_launches += static_cast<int>(iters);
             }
-            if (*s.host_len == 0) break;
+            if (over || *s.host_len == 0) break;  // (not over: a full chunk, whose last iteration fills queue 0)
             if (iter > max_iters) return cudaErrorLaunchFailure;  // cannot happen: every slot makes progress
         }
         t_site = "resolve";
-        k_mf_resolve<<<(npix + 255) / 256, 256, 0, stream>>>(fbuf, s, f0, frames, cam.exposure, p.spatial_denoise);
+        k_mf_resolve<<<(npix + 255) / 256, 256, 0, stream>>>(fbuf, s, frames_of, f0, frames, cam.exposure,
+                                                             p.spatial_denoise);
         ++nl;
     }
     if (launches) *launches = nl;
@@ -1355,16 +1356,14 @@ cudaError_t launch_render_batch(const DevScene &scene, const BatchParams &b, con
         for (;;) {
             for (uint32_t c = 0; c < kChunk; ++c) {
                 const int in = static_cast<int>(c & 1u), out = in ^ 1;
-                if ((e = cudaMemsetAsync(qc + out, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
-                const WavefrontState se =
+                        const WavefrontState se =
                     tuning.ray_sort ? enqueue_ray_sort(scene, s, in, counters, num_sms, stream) : s;
                 if ((e = launch_extend(scene, se, in, count, counters, extend_grid, stream, ev, true,
                                        c == 0 ? packet_forms : 0u)) != cudaSuccess)
                     return e;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                if (nee == kNeeDeferred && (e = reset_shadow_counters(counters, stream)) != cudaSuccess) return e;
-                shade<<<shade_blocks, 128, 0, stream>>>(scene, bg, ss, in, counters);
+                        shade<<<shade_blocks, 128, 0, stream>>>(scene, bg, ss, in, counters);
                 if (nee == kNeeDeferred)
                     enqueue_shadow_stage<2>(scene, DevCamera{}, FrameBuffers{}, RenderParams{}, bg, ss, b.rng, out, 0u,
                                             0u, counters, shadow_grid, shade_blocks, stream);

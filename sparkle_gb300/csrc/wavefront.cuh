@@ -39,9 +39,6 @@ struct WavefrontState {
     float4 *sample_normals = nullptr;         // multi-frame mode with the spatial fill: first-hit normal per sample
     size_t normal_capacity = 0;               // float4 entries of `sample_normals`
     // multi-frame mode: per-frame constants, frame k of the call
-    float *frame_weight = nullptr;      // DenoisePass moving-average weight of frame k
-    uint32_t *frame_seed = nullptr;     // dispatched sample count at frame k (per-pixel seed base)
-    uint32_t frame_capacity = 0;
     unsigned long long *host_len = nullptr;  // pinned: queue length read back between iteration chunks
     // Shadow stage of next-event estimation (allocated on first use, `nee_capacity` slots): the two
     // occlusion rays of a light-sampling vertex (k = 0 light, 1 sky) and the radiance each adds unoccluded.
@@ -95,6 +92,14 @@ struct ChunkGraph {
 };
 void chunk_graph_free(ChunkGraph &g);
 
+// Sample bookkeeping of the frames of one call (CameraRenderProxy.cpp:66-75, CPURenderer.cpp:206-207): frame k is
+// seeded with seed_base + k * spp and folded in with weight c / (c + spp), c = min(max_spp, cumulated + k * spp);
+// `clear`: the accumulation starts over (frame 0 folds into zeros).
+struct FrameSchedule {
+    uint32_t seed_base, spp, cumulated, max_spp;
+    bool clear;
+};
+
 // All `num_frames` frames of a call in one wavefront with path regeneration. Slots pull (frame, pixel) sample items
 // from a global counter in frame-major order; a slot whose path ends stores the sample's clamped result
 // and starts the next item, so every iteration keeps about one frame of paths in flight and only the
@@ -102,11 +107,12 @@ void chunk_graph_free(ChunkGraph &g);
 // frame order with each frame's weight (CPURenderer.cpp:530-543), so the frame buffer is bit-identical
 // to rendering the frames one by one. With the spatial DenoisePass on, every sample also keeps its first-hit
 // normal and the resolve applies the fill to each frame's samples before folding them (the fill reads only
-// the same frame's samples, so pixels still do not interact across frames). `weights[k]` / `seeds[k]` are
-// frame k's moving-average weight and seed base. Ends with the tonemap of the final frame buffer.
+// the same frame's samples, so pixels still do not interact across frames). `counters` must be zeroed. Ends with
+// the tonemap of the final frame buffer. A call of at most kFramesPerPass frames whose samples all start at once
+// returns without waiting for the GPU.
 cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam, const FrameBuffers &fbuf,
-                                     const RenderParams &p, uint32_t num_frames, const float *weights,
-                                     const uint32_t *seeds, bool count, Counters *counters, WavefrontState &s,
+                                     const RenderParams &p, uint32_t num_frames, const FrameSchedule &frames_of,
+                                     bool count, Counters *counters, WavefrontState &s,
                                      int num_sms, cudaStream_t stream, uint32_t *launches, LaunchEvents *ev,
                                      const WfTuning &tuning, ChunkGraph *graph);
 
