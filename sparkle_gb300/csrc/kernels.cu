@@ -13,19 +13,20 @@ namespace {
 // Ray-set query: persistent warps pull rays from a global counter and refill idle lanes.
 // ------------------------------------------------------------------------------------------------
 template <int kMode, bool kCount>
-__global__ void __launch_bounds__(128, SPK_WALK_MIN_BLOCKS) k_trace(DevScene S, const float *__restrict__ rays, uint64_t n,
+__global__ void __launch_bounds__(128, SPK_WALK_MIN_BLOCKS) k_trace(const __grid_constant__ DevScene S, const float *__restrict__ rays, uint64_t n,
                                                   spk_hit_dev *__restrict__ hits, Counters *counters) {
     uint32_t err = 0;
     TraceCounts tc;
-    walk_persistent<kMode, kCount>(
+    const uint32_t root = S.tlas_root;
+    walk_rays<kMode, kCount>(
         S, &counters->queue_counters[0], n, kFltMax, err, &tc,
-        [&](unsigned long long q, f3 &o, f3 &d, float &) {
+        [rays, root](unsigned long long q, f3 &o, f3 &d, float &) {
             const float *r = rays + q * 6;
             o = mk3(r[0], r[1], r[2]);
             d = mk3(r[3], r[4], r[5]);
-            return S.tlas_root;
+            return root;
         },
-        [&](unsigned long long q, const TraceResult &res) {
+        [hits](unsigned long long q, const TraceResult &res) {
             spk_hit_dev out;
             if (res.inst == kInvalid) {
                 out = spk_hit_dev{0.f, 0.f, 0.f, kInvalid, kInvalid};
@@ -159,9 +160,8 @@ cudaError_t launch_trace(const DevScene &scene, const float *rays, uint64_t n, v
                          Counters *counters, int num_sms, cudaStream_t stream, LaunchEvents *ev) {
     cudaError_t e = cudaMemsetAsync(&counters->queue_counters[0], 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
-    const uint64_t warps_needed = (n + 31) / 32;
-    uint64_t blocks = static_cast<uint64_t>(num_sms) * 12;  // persistent: ~12 blocks of 4 warps per SM
-    blocks = std::min<uint64_t>(blocks, (warps_needed + 3) / 4);
+    uint64_t blocks = static_cast<uint64_t>(num_sms) * SPK_WALK_MIN_BLOCKS;  // persistent: as many as are resident
+    blocks = std::min<uint64_t>(blocks, n);
     if (blocks == 0) blocks = 1;
     auto *h = static_cast<spk_hit_dev *>(hits);
     const unsigned g = static_cast<unsigned>(blocks);

@@ -33,6 +33,9 @@ enum : uint32_t { kErrStackOverflow = 1u, kErrIterationBudget = 2u, kErrQueueOve
 #ifndef SPK_REFILL_LANES
 #define SPK_REFILL_LANES 22  // persistent warps refill idle lanes once fewer than this are walking
 #endif
+#ifndef SPK_WIDE_RAYS_PER_BLOCK
+#define SPK_WIDE_RAYS_PER_BLOCK 12  // launches of at most this many rays per block walk one ray per warp
+#endif
 #ifndef SPK_TAIL_STEPS
 #define SPK_TAIL_STEPS 4  // steps between the rounds of a persistent warp that has no more rays to fetch
 #endif
@@ -293,36 +296,63 @@ __device__ __forceinline__ bool closer_hit(const TraceResult &best, float t, uin
     return t == best.t && (inst < best.inst || (inst == best.inst && face < best.face));
 }
 
-// Where a walk keeps its world ray. A one-thread walk: registers. A persistent walk: a column of the block's
-// shared memory (component k of thread t at [k][t]: any set of lanes reads its own or other lanes' rays without
-// bank conflicts), so that other lanes of the warp can test its triangles (TriangleQueue).
-struct RegWorld {
+// What a walk keeps but rarely touches: its world ray and where in its best triangle the hit is. A one-thread walk:
+// registers. A persistent walk: a column of the block's shared memory (word k of thread t at [k][t]: lanes that read
+// their own or distinct lanes' columns meet no bank conflict), so that other lanes of the warp can test its triangles
+// (TriangleQueue), and because the registers would spill in the node visit (two spilled words cost the walk 2-4%). 11
+// words a thread keep 7 blocks within a 64 KB shared-memory share of the SM; 14 words take the next share from the L1.
+struct RegState {
     f3 ro, rd;
-    __device__ __forceinline__ void set(f3 a, f3 b) {
+    float hit_u, hit_v;
+    uint32_t hit_face;
+    __device__ __forceinline__ void set_ray(f3 a, f3 b) {
         ro = a;
         rd = b;
     }
     __device__ __forceinline__ f3 o() const { return ro; }
     __device__ __forceinline__ f3 d() const { return rd; }
+    __device__ __forceinline__ void set_hit(float u, float v, uint32_t face) {
+        hit_u = u;
+        hit_v = v;
+        hit_face = face;
+    }
+    __device__ __forceinline__ float u() const { return hit_u; }
+    __device__ __forceinline__ float v() const { return hit_v; }
+    __device__ __forceinline__ uint32_t face() const { return hit_face; }
 };
-struct SharedWorld {
-    float *w;  // component 0 of this thread
-    __device__ __forceinline__ void set(f3 a, f3 b) {
+struct SharedState {
+    static constexpr int kWords = 11;
+    float *w;  // word 0 of this thread
+    __device__ __forceinline__ float &at(int k) const { return w[k * kWalkThreads]; }
+    __device__ __forceinline__ void set_ray(f3 a, f3 b) const {
         const float v[6] = {a.x, a.y, a.z, b.x, b.y, b.z};
 #pragma unroll
-        for (int k = 0; k < 6; ++k) w[k * kWalkThreads] = v[k];
+        for (int k = 0; k < 6; ++k) at(k) = v[k];
     }
-    __device__ __forceinline__ f3 o() const { return mk3(w[0], w[kWalkThreads], w[2 * kWalkThreads]); }
-    __device__ __forceinline__ f3 d() const {
-        return mk3(w[3 * kWalkThreads], w[4 * kWalkThreads], w[5 * kWalkThreads]);
+    __device__ __forceinline__ f3 o() const { return mk3(at(0), at(1), at(2)); }
+    __device__ __forceinline__ f3 d() const { return mk3(at(3), at(4), at(5)); }
+    __device__ __forceinline__ void set_hit(float u, float v, uint32_t face) const {
+        at(6) = u;
+        at(7) = v;
+        at(8) = __uint_as_float(face);
+    }
+    __device__ __forceinline__ float u() const { return at(6); }
+    __device__ __forceinline__ float v() const { return at(7); }
+    __device__ __forceinline__ uint32_t face() const { return __float_as_uint(at(8)); }
+    __device__ __forceinline__ void set_item(unsigned long long q) const {
+        at(9) = __uint_as_float(static_cast<uint32_t>(q));
+        at(10) = __uint_as_float(static_cast<uint32_t>(q >> 32));
+    }
+    __device__ __forceinline__ unsigned long long item() const {
+        return __float_as_uint(at(9)) | (static_cast<unsigned long long>(__float_as_uint(at(10))) << 32);
     }
 };
 
 // Resumable two-level walk of one ray. init() starts it; step() advances by one node visit and returns true when
-// the walk is over (result in `best`).
-template <int kMode, bool kCount, class World>
+// the walk is over (result in best()).
+template <int kMode, bool kCount, class State>
 struct Walker {
-    World world;
+    State st;
     LevelRay ray;
     uint2 ngroup;
     int sp;
@@ -330,11 +360,12 @@ struct Walker {
     uint32_t cur_inst;
     uint32_t steps_left;
     float tmax_box;
-    TraceResult best;
+    float best_t;
+    uint32_t best_inst;
 
     // `root` is the TLAS root node of the ray's scene (S.tlas_root for a single-scene context).
     __device__ __forceinline__ void init(const DevScene &S, uint32_t root, f3 o, f3 d, float tmax) {
-        world.set(o, d);
+        st.set_ray(o, d);
         setup_level(ray, o, d);
         ngroup = make_uint2(root, root == kInvalid ? 0u : (1u << 24));
         sp = 0;
@@ -342,7 +373,20 @@ struct Walker {
         cur_inst = 0;
         steps_left = S.walk_budget ? S.walk_budget : kMaxIterations;
         tmax_box = (kMode == kTraceOcclusion) ? tmax : kFltMax;
-        best = TraceResult{kFltMax, 0.f, 0.f, kInvalid, kInvalid};
+        best_t = kFltMax;
+        best_inst = kInvalid;
+        st.set_hit(0.f, 0.f, kInvalid);
+    }
+
+    __device__ __forceinline__ TraceResult best() const { return TraceResult{best_t, st.u(), st.v(), best_inst, st.face()}; }
+
+    // Takes the hit when it is closer than the best one (ties as closer_hit has them).
+    __device__ __forceinline__ bool take(float t, float u, float v, uint32_t inst, uint32_t face) {
+        if (!(t < best_t) && !(t == best_t && closer_hit(best(), t, inst, face))) return false;
+        best_t = t;
+        best_inst = inst;
+        st.set_hit(u, v, face);
+        return true;
     }
 
     template <class Stack>
@@ -365,7 +409,7 @@ struct Walker {
             if (I.type == 1u) {
                 // SphereRenderProxy::IntersectInternal (SphereRenderProxy.cpp:5-38), world space: sphere_hit's
                 // test, written out so the any-hit modes stop before the square root.
-                const f3 wo = world.o(), wd = world.d();
+                const f3 wo = st.o(), wd = st.d();
                 const f3 center = mk3(I.m[3], I.m[7], I.m[11]);
                 const f3 co = wo - center;
                 const float half_b = dot3(wd, co);
@@ -373,29 +417,26 @@ struct Walker {
                 const float disc = half_b * half_b - 1.f * c;
                 if (disc < 0.f) continue;
                 if (kMode == kTraceAnyRef) {
-                    best.inst = inst;
+                    best_inst = inst;
                     return true;
                 }
                 const float sq = sqrtf(disc);
                 const float t = (-half_b + (c >= 0.f ? -sq : sq)) / 1.f;
                 if (kMode == kTraceOcclusion) {
                     if (t > kEps && t < tmax_box) {
-                        best.inst = inst;
+                        best_inst = inst;
                         return true;
                     }
                     continue;
                 }
-                if (t > 0.f && closer_hit(best, t, inst, kInvalid)) {
-                    best = TraceResult{t, 0.f, 0.f, inst, kInvalid};
-                    tmax_box = prune_limit(best.t, wo.x, wd.x, S.scene_abs_x);
-                }
+                if (t > 0.f && take(t, 0.f, 0.f, inst, kInvalid)) tmax_box = prune_limit(t, wo.x, wd.x, S.scene_abs_x);
             } else if (I.blas_root != kInvalid) {
                 // Enter the BLAS: park the rest of this TLAS level on the stack.
                 if (tgroup.y != 0u) push(stack, tgroup, err);
                 if (ngroup.y > 0x00FFFFFFu) push(stack, ngroup, err);
                 blas_sp = sp;
                 cur_inst = inst;
-                setup_level(ray, xform_point(I.minv, world.o()), xform_dir(I.minv, world.d()));
+                setup_level(ray, xform_point(I.minv, st.o()), xform_dir(I.minv, st.d()));
                 ngroup = make_uint2(I.blas_root, 1u << 24);
                 tgroup.y = 0u;
             }
@@ -444,7 +485,7 @@ struct Walker {
             if (sp == blas_sp) blas_sp = -2;
             ngroup = stack.take(--sp);
             if (blas_sp == -2 && ngroup.y > 0x00FFFFFFu) {
-                setup_level(ray, world.o(), world.d());
+                setup_level(ray, st.o(), st.d());
                 blas_sp = -1;
             }
         }
@@ -457,7 +498,7 @@ template <int kMode, bool kCount = false>
 __device__ __forceinline__ TraceResult trace_ray(const DevScene &S, f3 wo, f3 wd, float tmax_occl, uint32_t &err,
                                                  TraceCounts *counts = nullptr) {
     LocalStack stack;
-    Walker<kMode, kCount, RegWorld> w;
+    Walker<kMode, kCount, RegState> w;
     w.init(S, S.tlas_root, wo, wd, tmax_occl);
     auto group = [&](uint2 tg) {
         while (tg.y != 0u) {
@@ -467,15 +508,12 @@ __device__ __forceinline__ TraceResult trace_ray(const DevScene &S, f3 wo, f3 wd
             uint32_t face;
             if (!triangle_hit(S.tris, idx, w.ray, t, u, v, face)) continue;
             if (kMode == kTraceAnyRef || (kMode == kTraceOcclusion && t < tmax_occl)) {
-                w.best.inst = w.cur_inst;
+                w.best_inst = w.cur_inst;
                 return true;
             }
             if (kMode == kTraceOcclusion) continue;
             const float wt = world_t(S.instances[w.cur_inst], w.ray, t, wo, wd);
-            if (wt > 0.f && closer_hit(w.best, wt, w.cur_inst, face)) {
-                w.best = TraceResult{wt, u, v, w.cur_inst, face};
-                w.tmax_box = prune_limit(wt, wo.x, wd.x, S.scene_abs_x);
-            }
+            if (wt > 0.f && w.take(wt, u, v, w.cur_inst, face)) w.tmax_box = prune_limit(wt, wo.x, wd.x, S.scene_abs_x);
         }
         return false;
     };
@@ -484,7 +522,7 @@ __device__ __forceinline__ TraceResult trace_ray(const DevScene &S, f3 wo, f3 wd
     };
     while (!w.step(S, stack, err, counts, leaves, group)) {
     }
-    return w.best;
+    return w.best();
 }
 
 // The triangles a warp's rays have reached and not tested yet: (triangle, instance) pairs with the lane that owns
@@ -522,18 +560,17 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
                                                 float tmax, uint32_t &err, TraceCounts *counts, Fetch &&fetch,
                                                 Finish &&finish) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
-    __shared__ float world[6 * kWalkThreads];
+    __shared__ float state[SharedState::kWords * kWalkThreads];
     __shared__ TriangleQueue queues[kWalkThreads / 32];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     TriangleQueue &Q = queues[threadIdx.x >> 5];
     LocalStack stack;
-    Walker<kMode, kCount, SharedWorld> w;
-    w.world.w = world + threadIdx.x;
+    Walker<kMode, kCount, SharedState> w;
+    w.st.w = state + threadIdx.x;
     bool walking = false, over = false;  // over: the walk has ended, its pairs may still be queued
     bool exhausted = false;
     uint32_t tail_steps = 0;
-    unsigned long long item = 0;
     if (lane == 0) Q.count = 0u;
     __syncwarp();
 
@@ -582,7 +619,7 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
             const uint2 e = Q.pair[lane];
             own = Q.owner[lane];
             inst = e.y;
-            const SharedWorld ow{world + (threadIdx.x & ~31u) + own};
+            const SharedState ow{state + (threadIdx.x & ~31u) + own};
             const DevInstance &I = S.instances[inst];
             const f3 wo = ow.o(), wd = ow.d();
             LevelRay r;
@@ -601,17 +638,14 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
                 const uint32_t o = __shfl_sync(kAll, own, src);
                 const TraceResult c{__shfl_sync(kAll, t, src), __shfl_sync(kAll, u, src), __shfl_sync(kAll, v, src),
                                     __shfl_sync(kAll, inst, src), __shfl_sync(kAll, face, src)};
-                if (o == lane && closer_hit(w.best, c.t, c.inst, c.face)) {
-                    w.best = c;
-                    closer = true;
-                }
+                if (o == lane && w.take(c.t, c.u, c.v, c.inst, c.face)) closer = true;
             }
-            if (closer) w.tmax_box = prune_limit(w.best.t, w.world.o().x, w.world.d().x, S.scene_abs_x);
+            if (closer) w.tmax_box = prune_limit(w.best_t, w.st.at(0), w.st.at(3), S.scene_abs_x);
         } else if (kMode == kTraceOcclusion) {
             const float limit = __shfl_sync(kAll, w.tmax_box, static_cast<int>(own));
             const uint32_t blocked = __reduce_or_sync(kAll, hit && t < limit ? 1u << own : 0u);
             if ((blocked >> lane) & 1u) {
-                w.best.inst = 0u;  // (which instance it was is not asked for)
+                w.best_inst = 0u;  // (which instance it was is not asked for)
                 over = over || walking;
                 walking = false;
             }
@@ -620,7 +654,7 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
                 const int src = __ffs(m) - 1;
                 const uint32_t o = __shfl_sync(kAll, own, src), ci = __shfl_sync(kAll, inst, src);
                 if (o == lane) {
-                    w.best.inst = ci;
+                    w.best_inst = ci;
                     over = over || walking;
                     walking = false;
                 }
@@ -645,15 +679,21 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
     for (;;) {
         const uint32_t idle = __ballot_sync(kAll, !walking && !over);
         if (!exhausted && idle != 0u) {
-            const uint32_t cnt = __popc(idle);
+            // A list of fewer than 32 rays per block is spread over as many warps as there are blocks, one fetch
+            // each: lanes of different warps do not wait for each other (335x202 pixels of the large scene: 1026 ->
+            // 947 us a frame; over all warps, four times as many, they crowd each other: 65536 rays of the box 28 ->
+            // 33 us).
+            const uint32_t quota = n < 32ull * gridDim.x ? static_cast<uint32_t>((n + gridDim.x - 1) / gridDim.x) : 32u;
+            const uint32_t cnt = min(static_cast<uint32_t>(__popc(idle)), quota);
             unsigned long long base = 0;
             if (lane == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(cnt));
             base = __shfl_sync(kAll, base, 0);
-            if (base + cnt >= n) exhausted = true;
+            exhausted = base + cnt >= n || quota < 32u;
             if (!walking && !over) {
-                const unsigned long long q = base + __popc(idle & lt_mask);
-                if (q < n) {
-                    item = q;
+                const uint32_t rank = __popc(idle & lt_mask);
+                const unsigned long long q = base + rank;
+                if (rank < cnt && q < n) {
+                    w.st.set_item(q);
                     f3 o, d;
                     float tm = tmax;
                     const uint32_t root = fetch(q, o, d, tm);
@@ -683,11 +723,212 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
                 round(cnt);
             }
             if (drain) {  // the queue is empty: every walk that is over has its result
-                if (over) finish(item, w.best);
+                if (over) finish(w.st.item(), w.best());
                 over = false;
                 if (!exhausted || walkers == 0u) break;
             }
         }
+    }
+}
+
+// Walk of few rays, one ray per warp: the warp visits up to four of the ray's nearest pending nodes at once, lane 8 g + k
+// testing child slot k ^ octant of node g (so that the ballot is in visiting order), and tests the triangles of the
+// leaves reached in the lanes that reached them. A launch of few rays lasts as long as its longest walk, whatever the
+// rest of the chip does: the last bounces of a 1080p frame (a few thousand rays) take hundreds of dependent steps. Here a
+// step is a few loads and some 60 instructions before the next ones are known, where walk_persistent's lane runs 250 and
+// visits one node. Same boxes (the plain slab test with a correctly rounded reciprocal), triangles and tie rule, so the
+// same results. `fetch` and `finish` as for walk_persistent; `finish` runs in one lane.
+// 4097 rays: 49 -> 22 us (11392 triangles). It takes 6 times the instructions per ray, so more rays soon do better with
+// a ray per lane: up to 12 rays per block (12768 on 152 SMs) it won or tied on all scenes, at 16 the 36-triangle box lost
+// 6% (its walks are short), at 8 a 10627-ray query of 200480 triangles took 117 us instead of 102.
+constexpr int kWideStack = 96;  // a step pushes at most 8 groups
+// Not inlined, so that its registers do not count against walk_persistent's in the same kernel. Returns error bits.
+template <int kMode, bool kCount, class Fetch, class Finish>
+__device__ __noinline__ uint32_t walk_wide(const DevScene &S, unsigned long long *cursor, unsigned long long n,
+                                           float tmax, TraceCounts *counts, Fetch fetch, Finish finish) {
+    uint32_t err = 0;
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, grp = lane >> 3;
+    uint2 stack[kWideStack];
+    for (;;) {
+        unsigned long long q = 0;
+        if (lane == 0) q = atomicAdd(cursor, 1ull);
+        q = __shfl_sync(kAll, q, 0);
+        if (q >= n) break;
+        f3 wo, wd;
+        float limit = tmax;  // boxes that start beyond it hold nothing closer; an occlusion walk's own limit
+        const uint32_t root = fetch(q, wo, wd, limit);
+        if (kMode != kTraceOcclusion) limit = kFltMax;
+        LevelRay ray;
+        setup_level<true>(ray, wo, wd);
+        TraceResult best{kFltMax, 0.f, 0.f, kInvalid, kInvalid};
+        uint2 ng = make_uint2(root, root == kInvalid ? 0u : (1u << 24));  // inner children in visiting order, or TLAS items
+        uint32_t left = S.walk_budget ? S.walk_budget : kMaxIterations;
+        uint32_t cur_inst = kInvalid;
+        int sp = 0, blas_sp = -1;  // blas_sp as in Walker
+        auto push = [&](uint2 g) {
+            if (sp < kWideStack) {
+                stack[sp++] = g;
+            } else {
+                err |= kErrStackOverflow;
+            }
+        };
+        for (bool done = ng.y == 0u; !done;) {
+            if (ng.y > 0x00FFFFFFu) {
+                const uint32_t inner = ng.y >> 24, imask = ng.y & 0xFFu;
+                const uint32_t cnt = sp + 8 <= kWideStack ? min(__popc(inner), 4) : 1;
+                if (left < cnt) {
+                    err |= kErrIterationBudget;
+                    break;
+                }
+                left -= cnt;
+                if (kCount && lane == 0) counts->nodes += cnt;
+                uint32_t rest = inner, mine = inner;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    if (k < grp && k + 1 < cnt) mine &= mine - 1u;  // (groups past `cnt` repeat its last node)
+                    if (k < cnt) rest &= rest - 1u;
+                }
+                const uint32_t parent_slot = (__ffs(mine) - 1) ^ ray.oct;
+                const uint32_t node = ng.x + __popc(imask & ((1u << parent_slot) - 1u));
+                if (rest != 0u) push(make_uint2(ng.x, (rest << 24) | imask));
+                const uint4 *np = S.nodes + static_cast<size_t>(node) * 5;
+                const uint4 n0 = __ldg(np), n1 = __ldg(np + 1);
+                const uint32_t slot = (lane & 7u) ^ ray.oct;
+                const uint8_t *lo = reinterpret_cast<const uint8_t *>(np + 2) + slot, *hi = lo + 24;
+                float tn[3], tf[3];
+                const float p[3] = {__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)};
+                const float ro[3] = {ray.o.x, ray.o.y, ray.o.z}, ri[3] = {ray.inv.x, ray.inv.y, ray.inv.z};
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const bool neg = (ray.oct >> k) & 1u;
+                    const float a = __uint_as_float(((n0.w >> (8 * k)) & 0xFFu) << 23) * ri[k];
+                    const float o = (p[k] - ro[k]) * ri[k];
+                    tn[k] = fmaf(static_cast<float>(__ldg((neg ? hi : lo) + 8 * k)), a, o);
+                    tf[k] = fmaf(static_cast<float>(__ldg((neg ? lo : hi) + 8 * k)), a, o);
+                }
+                const float t0 = fmaxf(fmaxf(tn[0], tn[1]), fmaxf(tn[2], 0.f));
+                const float t1 = fminf(fminf(tf[0], tf[1]), fminf(tf[2], limit));
+                const uint32_t meta = __byte_perm(n1.z, n1.w, slot) & 0xFFu;
+                const bool reached = grp < cnt && meta != 0u && t0 <= t1;
+                const bool leaf = (meta & 0x18u) != 0x18u;
+                const uint32_t inner_hits = __ballot_sync(kAll, reached && !leaf);
+                uint32_t items = reached && leaf ? (meta >> 5) << (meta & 31u) : 0u;
+                const bool in_blas = blas_sp >= 0;
+                if (in_blas) {
+                    // The lane's triangles (at most 3), then the closest over the warp.
+                    bool hit = false;
+                    float bt = kFltMax, bu = 0.f, bv = 0.f;
+                    uint32_t bface = kInvalid;
+                    if (kCount) counts->tris += __popc(items);
+                    while (__any_sync(kAll, items != 0u)) {
+                        if (items != 0u) {
+                            const uint32_t idx = n1.y + __ffs(items) - 1;
+                            items &= items - 1u;
+                            float t, u, v;
+                            uint32_t face;
+                            if (triangle_hit(S.tris, idx, ray, t, u, v, face)) {
+                                if (kMode == kTraceClosest) {
+                                    t = world_t(S.instances[cur_inst], ray, t, wo, wd);
+                                    if (t > 0.f && (t < bt || (t == bt && face < bface))) {
+                                        hit = true;
+                                        bt = t;
+                                        bu = u;
+                                        bv = v;
+                                        bface = face;
+                                    }
+                                } else {
+                                    hit = hit || kMode == kTraceAnyRef || t < limit;
+                                }
+                            }
+                        }
+                    }
+                    if (__any_sync(kAll, hit)) {
+                        if (kMode != kTraceClosest) {
+                            best.inst = cur_inst;
+                            break;
+                        }
+                        const uint32_t key = hit ? __float_as_uint(bt) : 0xFFFFFFFFu;  // t > 0: ordered as an integer
+                        const uint32_t first = __reduce_min_sync(kAll, key);
+                        const uint32_t face = __reduce_min_sync(kAll, key == first ? bface : kInvalid);
+                        const int src = __ffs(__ballot_sync(kAll, key == first && bface == face)) - 1;
+                        const TraceResult c{__uint_as_float(first), __shfl_sync(kAll, bu, src), __shfl_sync(kAll, bv, src),
+                                            cur_inst, face};
+                        if (closer_hit(best, c.t, c.inst, c.face)) {
+                            best = c;
+                            limit = prune_limit(best.t, wo.x, wd.x, S.scene_abs_x);
+                        }
+                    }
+                } else {  // the items of each TLAS node as one group
+#pragma unroll
+                    for (int d = 1; d < 8; d <<= 1) items |= __shfl_xor_sync(kAll, items, d);
+                }
+                // Farthest node's groups first onto the stack, the nearest node's last: it is taken next.
+                ng.y = 0u;
+                for (int g = static_cast<int>(cnt) - 1; g >= 0; --g) {
+                    const uint32_t hits = (inner_hits >> (8 * g)) & 0xFFu;
+                    const uint32_t base = __shfl_sync(kAll, n1.x, 8 * g), im = __shfl_sync(kAll, n0.w, 8 * g) >> 24;
+                    if (hits != 0u) {
+                        if (ng.y != 0u) push(ng);
+                        ng = make_uint2(base, (hits << 24) | im);
+                    }
+                    if (!in_blas) {
+                        const uint32_t ib = __shfl_sync(kAll, n1.y, 8 * g), bits = __shfl_sync(kAll, items, 8 * g);
+                        if (bits != 0u) {
+                            if (ng.y != 0u) push(ng);
+                            ng = make_uint2(ib, bits);
+                        }
+                    }
+                }
+            } else {  // TLAS items
+                const uint32_t inst = __ldg(S.tlas_items + ng.x + __ffs(ng.y) - 1);
+                ng.y &= ng.y - 1u;
+                const DevInstance &I = S.instances[inst];
+                if (I.type == 1u) {
+                    float t;
+                    if (kMode == kTraceClosest) {
+                        if (sphere_hit(I, wo, wd, t) && t > 0.f && closer_hit(best, t, inst, kInvalid)) {
+                            best = TraceResult{t, 0.f, 0.f, inst, kInvalid};
+                            limit = prune_limit(t, wo.x, wd.x, S.scene_abs_x);
+                        }
+                    } else if (sphere_hit(I, wo, wd, t) && (kMode == kTraceAnyRef || (t > kEps && t < limit))) {
+                        best.inst = inst;
+                        break;
+                    }
+                } else if (I.blas_root != kInvalid) {
+                    if (ng.y != 0u) push(ng);
+                    blas_sp = sp;
+                    cur_inst = inst;
+                    setup_level<true>(ray, xform_point(I.minv, wo), xform_dir(I.minv, wd));
+                    ng = make_uint2(I.blas_root, 1u << 24);
+                }
+            }
+            if (ng.y == 0u) {
+                if (sp == 0) break;
+                if (sp == blas_sp) blas_sp = -2;
+                ng = stack[--sp];
+                if (blas_sp == -2 && ng.y > 0x00FFFFFFu) {
+                    setup_level<true>(ray, wo, wd);
+                    blas_sp = -1;
+                }
+            }
+        }
+        if (lane == 0) finish(q, best);
+    }
+    return err;
+}
+
+// The walk of a launch's rays: one per warp while there are few, else persistent warps with a ray per lane.
+template <int kMode, bool kCount, class Fetch, class Finish>
+__device__ __forceinline__ void walk_rays(const DevScene &S, unsigned long long *cursor, unsigned long long n,
+                                          float tmax, uint32_t &err, TraceCounts *counts, Fetch &&fetch,
+                                          Finish &&finish) {
+    if (n <= static_cast<unsigned long long>(gridDim.x) * SPK_WIDE_RAYS_PER_BLOCK) {
+        TraceCounts c;
+        err |= walk_wide<kMode, kCount>(S, cursor, n, tmax, kCount ? &c : nullptr, fetch, finish);
+        if (kCount) *counts = c;
+    } else {
+        walk_persistent<kMode, kCount>(S, cursor, n, tmax, err, counts, fetch, finish);
     }
 }
 

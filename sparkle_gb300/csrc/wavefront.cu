@@ -243,7 +243,8 @@ template <bool kCount, bool kBatch = false, int kPackets = 0>
 __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
                                        : kPackets == 1 ? SPK_PACKET_MIN_BLOCKS
                                                        : SPK_WALK_MIN_BLOCKS)
-    k_wf_extend(DevScene S, WavefrontState s, int in_queue, Counters *counters) {
+    k_wf_extend(const __grid_constant__ DevScene S, const __grid_constant__ WavefrontState s, int in_queue,
+                Counters *counters) {
     // The stage's own resets, in place of memset nodes between the kernels: the queues the shade stage fills (nothing
     // reads them now). The shade stage zeroes the walks' cursors in turn.
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -261,12 +262,12 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
     uint32_t err = 0;
     TraceCounts tc;
     const uint32_t *queue = s.queue[in_queue] + first;
-    auto fetch = [&](unsigned long long q, f3 &o, f3 &d, float &) {
+    auto fetch = [&S, &s, queue](unsigned long long q, f3 &o, f3 &d, float &) {
         const uint32_t pid = queue[q];
         load_ray(s, pid, o, d);
         return kBatch ? s.slot_root[pid] : S.tlas_root;
     };
-    auto finish = [&](unsigned long long q, const TraceResult &h) {
+    auto finish = [&s, queue](unsigned long long q, const TraceResult &h) {
         const uint32_t pid = queue[q];
         s.hit[pid] = make_float4(h.t, h.u, h.v, __uint_as_float(h.inst));
         s.hit_face[pid] = h.face;
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
         walk_packets<kCount, kPackets>(S, &counters->queue_counters[kPackets == 2 ? kPacket2Cursor : kPacketCursor], n,
                                        err, &tc, fetch, finish);
     } else {
-        walk_persistent<kTraceClosest, kCount>(S, &counters->queue_counters[kCursor], n, kFltMax, err, &tc, fetch,
+        walk_rays<kTraceClosest, kCount>(S, &counters->queue_counters[kCursor], n, kFltMax, err, &tc, fetch,
                                                finish);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&counters->extension_rays, n);
@@ -767,13 +768,14 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_b_shade(DevScene 
 // (lane refill as in extend), then the in-order addition of the unoccluded radiance.
 // ------------------------------------------------------------------------------------------------
 template <bool kBatch>
-__global__ void __launch_bounds__(128, SPK_SHADOW_MIN_BLOCKS) k_wf_shadow(DevScene S, WavefrontState s,
+__global__ void __launch_bounds__(128, SPK_SHADOW_MIN_BLOCKS) k_wf_shadow(const __grid_constant__ DevScene S,
+                                                                       const __grid_constant__ WavefrontState s,
                                                                        Counters *counters) {
     uint32_t err = 0;
     const unsigned long long n = counters->queue_counters[kShadowLen];
-    walk_persistent<kTraceOcclusion, false>(
+    walk_rays<kTraceOcclusion, false>(
         S, &counters->queue_counters[kShadowCursor], n, kFltMax, err, nullptr,
-        [&](unsigned long long q, f3 &o, f3 &d, float &tmax) {
+        [&S, &s](unsigned long long q, f3 &o, f3 &d, float &tmax) {
             const uint32_t e = s.shadow_queue[q];
             const float4 o4 = s.shadow_o[e], d4 = s.shadow_d[e];
             o = mk3(o4.x, o4.y, o4.z);
@@ -781,7 +783,7 @@ __global__ void __launch_bounds__(128, SPK_SHADOW_MIN_BLOCKS) k_wf_shadow(DevSce
             tmax = o4.w;
             return kBatch ? s.slot_root[e >> 1] : S.tlas_root;
         },
-        [&](unsigned long long q, const TraceResult &h) {
+        [&s](unsigned long long q, const TraceResult &h) {
             if (h.inst == kInvalid) reinterpret_cast<float *>(s.nee_contrib + s.shadow_queue[q])[3] = 2.f;
         });
     if (err) atomicOr(&counters->error_flags, err);

@@ -1,6 +1,7 @@
-"""The persistent walk's triangle queue where it runs full: every ray of a warp reaches leaf after leaf of stacked
-triangles, up to 24 per node and lane against room for 64 per warp, so that most go back to the ray's stack and are
-queued again. Hits must equal the oracle's, at ray counts around a warp's 32 lanes."""
+"""Ray-set walks over stacked triangles, where every ray reaches leaf after leaf: few rays walk one per warp (three
+triangles per lane and step), more fill the persistent walk's triangle queue (up to 24 per node and lane against room
+for 64 per warp, so that most go back to the ray's stack and are queued again). Hits must equal the oracle's, at ray
+counts around a warp's 32 lanes, beside the largest one-per-warp launch (12 rays per block) and above it."""
 import numpy as np
 import pytest
 
@@ -32,7 +33,7 @@ def stacked_triangles(layers: int):
 
 
 @pytest.mark.parametrize("layers", [1, 24, 200])
-@pytest.mark.parametrize("count", [1, 31, 32, 33, 4097])
+@pytest.mark.parametrize("count", [1, 31, 32, 33, 4097, 12768, 12769, 34049])
 def test_stacked_triangles_match_the_oracle(layers, count):
     scene = stacked_triangles(layers)
     rng = np.random.default_rng(count)
