@@ -158,8 +158,6 @@ __global__ void __launch_bounds__(256) k_resolve(FrameBuffers fb, float f, float
 
 cudaError_t launch_trace(const DevScene &scene, const float *rays, uint64_t n, void *hits, int mode, bool count,
                          Counters *counters, int num_sms, cudaStream_t stream, LaunchEvents *ev) {
-    cudaError_t e = cudaMemsetAsync(&counters->queue_counters[0], 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
     uint64_t blocks = static_cast<uint64_t>(num_sms) * SPK_WALK_MIN_BLOCKS;  // persistent: as many as are resident
     blocks = std::min<uint64_t>(blocks, n);
     if (blocks == 0) blocks = 1;

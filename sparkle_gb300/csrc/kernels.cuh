@@ -113,7 +113,7 @@ struct RenderParams {
     uint32_t enable_nee;
 };
 
-// Ray-set query over spk_ray records (24 B) into spk_hit records (20 B).
+// Ray-set query over spk_ray records (24 B) into spk_hit records (20 B). `counters` must be zeroed.
 cudaError_t launch_trace(const DevScene &scene, const float *rays, uint64_t n, void *hits, int mode, bool count,
                          Counters *counters, int num_sms, cudaStream_t stream, LaunchEvents *ev);
 
