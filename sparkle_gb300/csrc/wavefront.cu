@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <vector>
 
 #include "wavefront.cuh"
 #include "fault.h"
@@ -114,11 +115,15 @@ enum : int { kNeeOff = 0, kNeeInline = 1, kNeeDeferred = 2 };
 // next-event estimation at diffuse-branch vertices with MIS on the emission the BSDF rays collect.
 // kNeeInline walks the two occlusion rays here; kNeeDeferred stores them with their radiance for the
 // shadow stage and returns in `nee_rays` which were queued (bit k: ray k), the colour still without them.
-// Returns whether the path continues (the next ray is then in s.ray_a / s.ray_b).
-template <int kKind, int kNee>
+// Returns whether the path continues (the next ray is then in s.ray_a / s.ray_b); `result` is its radiance and valid
+// flag so far. Without NEE only a path's last segment adds radiance (sky or emission), so s.color is neither read nor
+// written here: the caller stores `result` where it wants the sample of a path that ended (32 of some 216 bytes per
+// segment; the stage is bound by this traffic). `first_normals` (spatial fill) takes the first hit's normal at
+// s.slot_item[pid] (kItemNormals) or pid.
+template <int kKind, int kNee, bool kItemNormals>
 __device__ __forceinline__ bool shade_path(const DevScene &S, const WavefrontState &s, uint32_t pid,
-                                           uint32_t bounce, float4 *gnormal, uint32_t &shadow, uint32_t &err,
-                                           uint32_t &nee_rays, size_t gnormal_index) {
+                                           uint32_t bounce, float4 *first_normals, uint32_t &shadow, uint32_t &err,
+                                           uint32_t &nee_rays, float4 &result) {
     constexpr bool nee = kNee != kNeeOff;
     nee_rays = 0u;
     bool alive = false;
@@ -128,7 +133,7 @@ __device__ __forceinline__ bool shade_path(const DevScene &S, const WavefrontSta
     load_ray(s, pid, o, d);
     // A path's first segment starts from throughput 1, colour 0, valid flag 1 and no light-sampling pdf
     // (start_path leaves them unstored).
-    const float4 c4 = bounce == 0 ? make_float4(0.f, 0.f, 0.f, 1.f) : s.color[pid];
+    const float4 c4 = !nee || bounce == 0 ? make_float4(0.f, 0.f, 0.f, 1.f) : s.color[pid];
     f3 color = mk3(c4.x, c4.y, c4.z);
     const float4 t4 = bounce == 0 ? make_float4(1.f, 1.f, 1.f, 0.f) : s.thr[pid];
     f3 thr = mk3(t4.x, t4.y, t4.z);
@@ -144,8 +149,8 @@ __device__ __forceinline__ bool shade_path(const DevScene &S, const WavefrontSta
         const TraceResult h{hit4.x, hit4.y, hit4.z, inst, s.hit_face[pid]};
         const Surface surf = make_surface(S, h, o, d);
         const DevMaterial mat = resolve_material(S, S.materials[surf.material], surf.uv);
-        if (bounce == 0 && gnormal)
-            gnormal[gnormal_index] = make_float4(surf.normal.x, surf.normal.y, surf.normal.z, 0.f);
+        if (bounce == 0 && first_normals)
+            first_normals[kItemNormals ? s.slot_item[pid] : pid] = make_float4(surf.normal.x, surf.normal.y, surf.normal.z, 0.f);
         if (mat.is_emissive) {
             f3 c = cmul(mk3(mat.emissive[0], mat.emissive[1], mat.emissive[2]), thr);
             if (prev_pdf > 0.f) c = c * bsdf_hit_weight(S, prev_pdf, h, d);
@@ -208,7 +213,8 @@ __device__ __forceinline__ bool shade_path(const DevScene &S, const WavefrontSta
             s.thr[pid] = make_float4(thr.x, thr.y, thr.z, 0.f);
         }
     }
-    s.color[pid] = make_float4(color.x, color.y, color.z, valid);
+    result = make_float4(color.x, color.y, color.z, valid);
+    if (nee) s.color[pid] = result;
     return alive;
 }
 
@@ -287,6 +293,33 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
     if (err) atomicOr(&counters->error_flags, err);
 }
 
+// The shade stages' threads per block.
+constexpr uint32_t kShadeThreads = 128;
+
+// Takes the block's next kShadeThreads queue entries (kInvalid past the end) and hands them out with the paths that hit
+// something first, the order otherwise kept: a path that missed only looks the sky up, and mixed with those that hit it
+// left the long part of shading 11 of 32 lanes (secondary rays of the terrain scene, 60% misses). Every thread calls it.
+__device__ __forceinline__ uint32_t hits_first(const WavefrontState &s, uint32_t pid) {
+    __shared__ uint32_t order[kShadeThreads];
+    __shared__ uint32_t warp_hits[kShadeThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const bool hit = pid != kInvalid && __float_as_uint(s.hit[pid].w) != kInvalid;
+    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, hit);
+    if (lane == 0) warp_hits[warp] = __popc(mask);
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kShadeThreads / 32; ++k) {
+        if (k < warp) before += warp_hits[k];
+        total += warp_hits[k];
+    }
+    before += __popc(mask & ((1u << lane) - 1u));  // hits before this thread
+    order[hit ? before : total + threadIdx.x - before] = pid;
+    __syncthreads();
+    pid = order[threadIdx.x];
+    return pid;
+}
+
 // After an extend stage: its cursors back to zero, and no packet prefix (the next queue is mixed).
 __device__ __forceinline__ void reset_walk(Counters *counters) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -310,14 +343,17 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_wf_shade(DevScene
          q0 += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
         const unsigned long long q = q0 + threadIdx.x;
         bool alive = false;
-        uint32_t pid = 0, nee_rays = 0;
-        if (q < n) {
-            pid = queue[q];
-            alive = shade_path<kKind, kNee>(S, s, pid, bounce, p.spatial_denoise ? fb.gnormal : nullptr, shadow, err,
-                                             nee_rays, pid);
+        uint32_t pid = q < n ? queue[q] : kInvalid, nee_rays = 0;
+        if (bounce != 0) pid = hits_first(s, pid);
+        if (pid != kInvalid) {
+            float4 result;
+            alive = shade_path<kKind, kNee, false>(S, s, pid, bounce, p.spatial_denoise ? fb.gnormal : nullptr, shadow,
+                                                   err, nee_rays, result) &&
+                    bounce + 1 < p.bounce;
+            if (kNee == kNeeOff && !alive) s.color[pid] = result;
         }
         if constexpr (kNee == kNeeDeferred) queue_nee(s, counters, pid, nee_rays, false);
-        queue_push(s.queue[out_queue], &counters->queue_counters[out_queue], pid, alive && bounce + 1 < p.bounce);
+        queue_push(s.queue[out_queue], &counters->queue_counters[out_queue], pid, alive);
     }
     warp_add_u64(&counters->shadow_rays, shadow);
     if (err) atomicOr(&counters->error_flags, err);
@@ -404,12 +440,13 @@ __global__ void __launch_bounds__(128) k_mf_generate(DevCamera cam, FrameBuffers
     }
 }
 
-// Shade one segment per live slot. A finished sample stores its clamped result (RenderPixel's 6.0 clamp,
+// Shade one segment per live slot (`common_bounce`: every path's segment when all started together, -1 when each slot
+// has its own in slot_state). A finished sample stores its clamped result (RenderPixel's 6.0 clamp,
 // CPURenderer.cpp:408) at its item, and the slot takes the next item from the global counter.
 template <int kKind, int kNee>
 __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_mf_shade(DevScene S, DevCamera cam, FrameBuffers fb, RenderParams p,
                                                   WavefrontState s, int in_queue, uint32_t frame_base,
-                                                  uint32_t total_items, Counters *counters) {
+                                                  uint32_t total_items, int common_bounce, Counters *counters) {
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
@@ -420,18 +457,18 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_mf_shade(DevScene
          q0 += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
         const unsigned long long q = q0 + threadIdx.x;
         bool push = false, need = false, alive = false;
-        uint32_t slot = 0, nee_rays = 0;
-        if (q < n) {
-            slot = queue[q];
-            const uint32_t bounce = s.slot_state[slot];
-            alive = shade_path<kKind, kNee>(S, s, slot, bounce, p.spatial_denoise ? s.sample_normals : nullptr, shadow,
-                                            err, nee_rays, s.slot_item[slot]) &&
+        uint32_t slot = q < n ? queue[q] : kInvalid, nee_rays = 0;
+        if (common_bounce != 0) slot = hits_first(s, slot);
+        if (slot != kInvalid) {
+            const uint32_t bounce = common_bounce >= 0 ? static_cast<uint32_t>(common_bounce) : s.slot_state[slot];
+            float4 c;
+            alive = shade_path<kKind, kNee, true>(S, s, slot, bounce, p.spatial_denoise ? s.sample_normals : nullptr,
+                                                  shadow, err, nee_rays, c) &&
                     bounce + 1 < p.bounce;
             if (alive) {
-                s.slot_state[slot] = bounce + 1u;
+                if (common_bounce < 0) s.slot_state[slot] = bounce + 1u;
                 push = true;
             } else if (nee_rays == 0u) {
-                const float4 c = s.color[slot];
                 s.samples[s.slot_item[slot]] =
                     make_float4(clamp_sample(c.x), clamp_sample(c.y), clamp_sample(c.z), c.w);
                 need = true;
@@ -725,19 +762,18 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_b_shade(DevScene 
          q0 += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
         const unsigned long long q = q0 + threadIdx.x;
         bool push = false, need = false, alive = false;
-        uint32_t slot = 0, nee_rays = 0;
-        if (q < n) {
-            slot = queue[q];
+        uint32_t slot = hits_first(s, q < n ? queue[q] : kInvalid), nee_rays = 0;
+        if (slot != kInvalid) {
             const DevRequest &R = b.reqs[s.slot_req[slot]];
             const DevScene Sv = scene_view(S, S.descs[R.scene]);
             const uint32_t bounce = s.slot_state[slot];
-            alive = shade_path<kKind, kNee>(Sv, s, slot, bounce, nullptr, shadow, err, nee_rays, 0) &&
+            float4 c;
+            alive = shade_path<kKind, kNee, true>(Sv, s, slot, bounce, nullptr, shadow, err, nee_rays, c) &&
                     bounce + 1 < R.bounce;
             if (alive) {
                 s.slot_state[slot] = bounce + 1u;
                 push = true;
             } else if (nee_rays == 0u) {
-                const float4 c = s.color[slot];
                 s.samples[s.slot_item[slot]] = make_float4(clamp_sample(c.x), clamp_sample(c.y), clamp_sample(c.z), c.w);
                 need = true;
             }
@@ -957,7 +993,7 @@ WfShadeFn pick_wf_shade(uint32_t rng, int nee) {
     return nee == kNeeOff ? k_wf_shade<1, kNeeOff> : nee == kNeeInline ? k_wf_shade<1, kNeeInline> : k_wf_shade<1, kNeeDeferred>;
 }
 
-using MfShadeFn = void (*)(DevScene, DevCamera, FrameBuffers, RenderParams, WavefrontState, int, uint32_t, uint32_t,
+using MfShadeFn = void (*)(DevScene, DevCamera, FrameBuffers, RenderParams, WavefrontState, int, uint32_t, uint32_t, int,
                            Counters *);
 MfShadeFn pick_mf_shade(uint32_t rng, int nee) {
     if (rng == 0) return nee == kNeeOff ? k_mf_shade<0, kNeeOff> : nee == kNeeInline ? k_mf_shade<0, kNeeInline> : k_mf_shade<0, kNeeDeferred>;
@@ -1072,6 +1108,7 @@ cudaError_t launch_render_wavefront(const DevScene &scene, const DevCamera &cam,
         k_wf_generate<1><<<ggrid, 128, 0, stream>>>(cam, fbuf, p, s, counters);
     }
     ++nl;
+    auto *shade = pick_wf_shade(p.rng, nee);
     const unsigned shade_blocks = static_cast<unsigned>(num_sms) * tuning.shade_blocks_per_sm;
     const unsigned extend_grid = extend_blocks(num_sms, tuning.extend_blocks_per_sm);
     const unsigned shadow_grid = shadow_blocks(num_sms, tuning.extend_blocks_per_sm);
@@ -1090,7 +1127,7 @@ cudaError_t launch_render_wavefront(const DevScene &scene, const DevCamera &cam,
             ss = enqueue_material_sort(scene, se, in, counters, num_sms, stream);
             nl += 3;
         }
-        pick_wf_shade(p.rng, nee)<<<shade_blocks, 128, 0, stream>>>(scene, fbuf, p, ss, in, b, counters);
+        shade<<<shade_blocks, 128, 0, stream>>>(scene, fbuf, p, ss, in, b, counters);
         ++nl;
         if (nee == kNeeDeferred) {
             enqueue_shadow_stage<0>(scene, cam, fbuf, p, BatchParams{}, ss, p.rng, out, 0u, 0u, counters, shadow_grid,
@@ -1140,6 +1177,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
         s.normal_capacity = need;
     }
     unsigned long long *qc = counters->queue_counters;
+    auto *shade = pick_mf_shade(p.rng, nee);
     const unsigned shade_blocks = static_cast<unsigned>(num_sms) * tuning.shade_blocks_per_sm;
     const unsigned extend_grid = extend_blocks(num_sms, tuning.extend_blocks_per_sm);
     const unsigned shadow_grid = shadow_blocks(num_sms, tuning.extend_blocks_per_sm);
@@ -1161,6 +1199,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
         // no more are launched than that, and the queue length need not be read back to know that they are over.
         const bool at_once = initial == total_items;
         const uint32_t iters = at_once ? std::min(p.bounce, kChunk) : kChunk;
+        const bool together = at_once && p.bounce <= kChunk;  // iteration c shades every path's segment c
         ++nl;
         // One chunk: `iters` iterations of (extend, shade).
         auto enqueue_chunk = [&](LaunchEvents *chunk_ev) -> cudaError_t {
@@ -1174,8 +1213,8 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                     return ce;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                pick_mf_shade(p.rng, nee)<<<shade_blocks, 128, 0, stream>>>(scene, cam, fbuf, p, ss, in, f0,
-                                                                            total_items, counters);
+                shade<<<shade_blocks, 128, 0, stream>>>(
+                    scene, cam, fbuf, p, ss, in, f0, total_items, together ? static_cast<int>(c) : -1, counters);
                 if (nee == kNeeDeferred)
                     enqueue_shadow_stage<1>(scene, cam, fbuf, p, BatchParams{}, ss, p.rng, out, f0, total_items,
                                             counters, shadow_grid, shade_blocks, stream);
@@ -1196,7 +1235,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                 uint32_t f0, total_items, count, num_sms;
                 Counters *counters;
                 cudaStream_t stream;
-                unsigned extend_grid, shade_grid, material_sort, ray_sort, nee_mode, packet_forms, iters;
+                unsigned extend_grid, shade_grid, material_sort, ray_sort, nee_mode, packet_forms, iters, together;
             } key;
             std::memset(static_cast<void *>(&key), 0, sizeof(key));  // padding too: the key is compared bytewise
             key.scene = scene;
@@ -1217,6 +1256,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
             key.nee_mode = static_cast<unsigned>(nee);
             key.packet_forms = packet_forms;
             key.iters = iters;
+            key.together = together ? 1u : 0u;
             const auto *kb = reinterpret_cast<const unsigned char *>(&key);
             graph_ev.pairs = graph->events;
             graph_ev.capacity = static_cast<int>(kChunk);
@@ -1325,11 +1365,11 @@ cudaError_t launch_render_batch(const DevScene &scene, const BatchParams &b, con
     const int nee = nee_mode(b.enable_nee, tuning);
     if (nee == kNeeDeferred && (e = wavefront_alloc_nee(s)) != cudaSuccess) return e;
     unsigned long long *qc = counters->queue_counters;
+    auto *shade = pick_b_shade(b.rng, nee);
     const unsigned shade_blocks = static_cast<unsigned>(num_sms) * tuning.shade_blocks_per_sm;
     const unsigned extend_grid = extend_blocks(num_sms, tuning.extend_blocks_per_sm);
     const unsigned shadow_grid = shadow_blocks(num_sms, tuning.extend_blocks_per_sm);
     const unsigned long long want = tuning.batch_slots ? tuning.batch_slots : s.capacity;
-    auto *shade = pick_b_shade(b.rng, nee);
     constexpr uint32_t kChunk = kChunkIterations;
     for (const BatchGroup &grp : groups) {
         if (grp.item_hi <= grp.item_lo || grp.item_hi > b.total_items) return cudaErrorInvalidValue;
