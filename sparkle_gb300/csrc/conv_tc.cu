@@ -1,19 +1,21 @@
 // conv_tc.cu -- tcgen05 implicit-GEMM 3x3 convolutions (see conv_tc.cuh).
 //
 // Forward / dgrad (one CTA per output tile of tw x (mt * th) pixels: mt M tiles of tw x th = 128 pixels
-// stacked vertically, tw a multiple of 8, 4 warps):
+// stacked vertically, tw a multiple of 8, 8 warps):
 //   warp 0 lane 0  TMA producer: per K block (column tap dx, 32-channel chunk) one 4-D tiled load of the
 //                  input box {32 ch, tw px, mt * th + 2 rows, 1 image} shifted by dx and reaching one row
 //                  above and below the tile (zero fill outside the image = the conv's padding), and three
 //                  2-D loads of the weight slices {32, cout} of the taps (dy, dx), dy = -1, 0, 1, into a
 //                  ring of 2-4 stages;
-//   warp 1 lane 0  MMA issuer: per stage, row tap dy and M tile m, two kind::f16 MMAs (K = 16 each) whose A
+//   warp 1         MMA issuer: per stage, row tap dy and M tile m, two kind::f16 MMAs (K = 16 each) whose A
 //                  operand starts (m * th + dy + 1) * tw rows into the input box -- a whole number of 8-row
 //                  swizzle atoms, so one box serves all three row taps of all M tiles and one weight slice
 //                  serves all M tiles -- into M tile m's 128 x cout FP32 accumulator in TMEM (columns
 //                  m * cout ...), committing each stage back to the producer;
-//   all 4 warps    epilogue: tcgen05.ld of the pixel rows (warp w owns TMEM lanes 32w..32w+31), bias,
+//   all warps      epilogue: tcgen05.ld of the pixel rows (warp w owns TMEM lanes 32w..32w+31), bias,
 //                  ReLU or ReLU-backward mask, BF16 pack, 16-byte stores.
+// Layers whose weights fit beside the ring, on images of several tiles per SM, go to k_conv_res instead: the
+// same MMAs from persistent CTAs that keep the weights.
 // Wgrad (one CTA per (128 rows of (tap, ci), pixel range)): TMA loads of the shifted input and the output
 // gradient as they lie in NHWC memory (MN-major operands, 64-byte swizzle), MMAs that read them MN-major,
 // and the FP32 partial sums added to dw with atomics. (SPK_CONV_WGRAD_TMA=0 keeps the earlier form: all
@@ -212,31 +214,30 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             for (uint32_t dy3 = 0; dy3 < 3; ++dy3)
                 tma_load_2d(b + dy3 * b_bytes, &tmw, &full[s], static_cast<int>((dy3 * 3u + dx3) * P.cin + c * 32u), 0);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         const uint32_t idesc = idesc_bf16(kTileM, P.cout);
+        const bool issue = elect_one();
         bool ok = true;
         for (uint32_t kb = 0; kb < nk; ++kb) {
             const uint32_t s = kb % nst, u = kb / nst;
-            if (!mbar_wait(&full[s], u & 1u, P.err)) {
-                ok = false;
-                break;
-            }
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], u & 1u, P.err));
+            if (!ok) break;
             tc_fence_after();
-            const uint32_t a = smem_u32(smem + s * stage_bytes), b = a + P.a_bytes;
+            const uint32_t a = smem_desc_sw64(smem_u32(smem + s * stage_bytes));
+            const uint32_t b = a + P.a_bytes / 16u;
+            const uint32_t row = P.tw * 4u, m_step = P.th * row;  // 64 bytes a pixel, in 16-byte units
 #pragma unroll
             for (uint32_t dy3 = 0; dy3 < 3; ++dy3) {
-                const uint32_t bd = b + dy3 * b_bytes;
                 for (uint32_t m = 0; m < P.mt; ++m) {
-                    const uint32_t ad = a + (m * P.th + dy3) * P.tw * 64u;
 #pragma unroll
                     for (uint32_t k2 = 0; k2 < 2; ++k2)
-                        mma_bf16(tmem + m * P.cout, smem_desc_sw64(ad + 32u * k2), smem_desc_sw64(bd + 32u * k2),
-                                 idesc, (kb | dy3 | k2) != 0u);
+                        mma_bf16(tmem + m * P.cout, a + m * m_step + dy3 * row + 2u * k2, kDescHiSw64,
+                                 b + dy3 * (b_bytes / 16u) + 2u * k2, kDescHiSw64, idesc, kb | dy3 | k2, issue);
                 }
             }
-            mma_commit(&empty[s]);
+            mma_commit(&empty[s], issue);
         }
-        if (ok) mma_commit(accum);
+        if (ok) mma_commit(accum, issue);
     }
     __syncwarp();
 
@@ -292,6 +293,203 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             tma_store_commit();
             tma_store_wait_read();
         }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, ncols);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Forward with resident weights
+// ------------------------------------------------------------------------------------------------
+// Persistent CTAs over tiles of 16 x 16 pixels (two M tiles of 16 x 8, stacked). All 9 * cin * cout weights of
+// the layer stay in shared memory. A ring of input boxes and two sets of accumulators let the loads of one
+// tile run under the MMAs and the epilogue of the tiles before it:
+//   warps 0-7  epilogue, four per M tile;
+//   warp 8     MMA issuer, which also loads the weights at the start;
+//   warp 9     input boxes by TMA, one per K block (column tap, channel chunk), as in k_conv_fwd.
+// K blocks, row taps and half chunks run in k_conv_fwd's order: the sums are the same bit for bit.
+// What k_conv_fwd spends most of a narrow layer on is each CTA's set-up, first load and epilogue, one after the
+// other: without any MMA a 32 -> 32 layer of 1920 x 1088 took 82 of its 88 us. Here they overlap: 59 us, 4.5
+// TB/s of input and output. What is left is mostly the MMAs' reads of A (128 rows of 32 bytes for 32 columns
+// of output, about 55 cycles each). 64 -> 64 at 960 x 544: 54.7 -> 37.9 us. Input boxes stored once per chunk
+// as planes without swizzle, where all nine taps are start addresses, were slower (91 us): the MMA reads such
+// a box at about 80 cycles each.
+constexpr uint32_t kResTile = 16;  // tile side
+constexpr uint32_t kResM = 2;      // M tiles
+constexpr uint32_t kResMRows = kResTile / kResM;
+constexpr uint32_t kResBoxBytes = fwd_a_bytes(kResTile, kResTile);
+constexpr uint32_t kResEpiWarps = 4 * kResM;
+constexpr uint32_t kResThreads = 32u * (kResEpiWarps + 2u);
+constexpr uint32_t kResStages = 6;  // input boxes at most
+constexpr uint32_t kResCtas = 2;    // CTAs per SM at most
+constexpr uint32_t kResBars = 256;
+
+struct ResParams {
+    uint32_t n, h, w, cin, cout;
+    uint32_t tiles_x, tiles_y, tiles, stages;
+    OutSpec out_spec;
+    uint32_t *err;
+};
+
+// Shared memory: weights, the staged outputs, the ring, the bias, barriers; 1 KB for the alignment.
+__host__ __device__ constexpr uint32_t res_weight_bytes(uint32_t cin, uint32_t cout) { return 18u * cin * cout; }
+__host__ __device__ constexpr uint32_t res_smem_bytes(uint32_t cin, uint32_t cout, uint32_t stages) {
+    return res_weight_bytes(cin, cout) + 2u * kResM * kTileM * cout + stages * kResBoxBytes + 4u * cout + kResBars +
+           1024u;
+}
+
+template <bool kPool>
+__global__ void __launch_bounds__(kResThreads, kResCtas)
+    k_conv_res(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw,
+               const __grid_constant__ CUtensorMap tmy, ResParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *wsm = align1024(smem_raw);
+    uint8_t *staged = wsm + res_weight_bytes(P.cin, P.cout);
+    uint8_t *ring = staged + 2u * kResM * kTileM * P.cout;
+    const uint32_t nst = P.stages;
+    float *bias = reinterpret_cast<float *>(ring + nst * kResBoxBytes);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(bias + P.cout);
+    uint64_t *full = bars, *empty = bars + kResStages, *acc_full = bars + 2 * kResStages,
+             *acc_empty = acc_full + 2, *wfull = acc_full + 4;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 5);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t acc_cols = kResM * P.cout, ncols = tmem_columns(2u * acc_cols);
+    const uint32_t nch = P.cin / 32u, nk = 3u * nch, b_bytes = P.cout * 64u;
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < nst; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (uint32_t s = 0; s < 2; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 32u * kResEpiWarps);
+        }
+        mbar_init(wfull, 1);
+        fence_mbar_init();
+    }
+    if (warp == 0) tmem_alloc(tmem_slot, ncols);
+    if (threadIdx.x < P.cout) bias[threadIdx.x] = P.out_spec.bias ? P.out_spec.bias[threadIdx.x] : 0.f;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const uint32_t my_tiles = (P.tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x;  // gridDim.x <= tiles
+
+    if (warp == kResEpiWarps + 1u) {
+        if (lane == 0) {
+            tma_prefetch_desc(&tmx);
+            uint32_t s = 0, u = 0;  // stage, and how often the ring has wrapped
+            bool ok = true;
+            for (uint32_t i = 0; ok && i < my_tiles; ++i) {
+                uint32_t q = blockIdx.x + i * gridDim.x;
+                const int x0 = static_cast<int>((q % P.tiles_x) * kResTile) - 1;
+                q /= P.tiles_x;
+                const int y0 = static_cast<int>((q % P.tiles_y) * kResTile) - 1;
+                const int img = static_cast<int>(q / P.tiles_y);
+                for (uint32_t dx3 = 0; ok && dx3 < 3; ++dx3)
+                    for (uint32_t c = 0; c < nch; ++c) {
+                        ok = u == 0 || mbar_wait(&empty[s], (u - 1) & 1u, P.err);
+                        if (!ok) break;
+                        mbar_arrive_expect_tx(&full[s], 64u * kResTile * (kResTile + 2u));
+                        tma_load_4d(ring + s * kResBoxBytes, &tmx, &full[s], static_cast<int>(c * 32u),
+                                    x0 + static_cast<int>(dx3), y0, img);
+                        if (++s == nst) s = 0, ++u;
+                    }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kResEpiWarps) {
+        const bool issue = elect_one();
+        if (issue) {
+            tma_prefetch_desc(&tmy);
+            mbar_arrive_expect_tx(wfull, res_weight_bytes(P.cin, P.cout));
+            for (uint32_t k = 0; k < 9u * nch; ++k)
+                tma_load_2d(wsm + k * b_bytes, &tmw, wfull, static_cast<int>(k * 32u), 0);
+        }
+        __syncwarp();
+        const uint32_t idesc = idesc_bf16(kTileM, P.cout);
+        const uint32_t wdesc = smem_desc_sw64(smem_u32(wsm)), ring_desc = smem_desc_sw64(smem_u32(ring));
+        const uint32_t b_step = b_bytes / 16u;
+        constexpr uint32_t row = kResTile * 4u;  // one row of a box, in 16-byte units
+        uint32_t s = 0, u = 0;
+        bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(wfull, 0, P.err));
+        for (uint32_t i = 0; ok && i < my_tiles; ++i) {
+            const uint32_t set = i & 1u, v = i >> 1, d = tmem + set * acc_cols;
+            ok = __all_sync(0xFFFFFFFFu, v == 0 || mbar_wait(&acc_empty[set], (v - 1) & 1u, P.err));
+            for (uint32_t kb = 0; ok && kb < nk; ++kb) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], u & 1u, P.err));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t a = ring_desc + s * (kResBoxBytes / 16u), b = wdesc + kb * b_step;
+#pragma unroll
+                for (uint32_t dy3 = 0; dy3 < 3; ++dy3)
+#pragma unroll
+                    for (uint32_t m = 0; m < kResM; ++m)
+#pragma unroll
+                        for (uint32_t k2 = 0; k2 < 2; ++k2)
+                            mma_bf16(d + m * P.cout, a + (m * kResMRows + dy3) * row + 2u * k2, kDescHiSw64,
+                                     b + dy3 * nk * b_step + 2u * k2, kDescHiSw64, idesc, kb | dy3 | k2, issue);
+                mma_commit(&empty[s], issue);
+                if (++s == nst) s = 0, ++u;
+            }
+            if (ok) mma_commit(&acc_full[set], issue);
+        }
+        __syncwarp();
+    } else {
+        const uint32_t m = warp >> 2, r = threadIdx.x & (kTileM - 1u);  // M tile; its pixel = TMEM lane
+        uint8_t *out_tile = staged + m * 2u * kTileM * P.cout;
+        for (uint32_t i = 0; i < my_tiles; ++i) {
+            const uint32_t set = i & 1u;
+            uint32_t q = blockIdx.x + i * gridDim.x;
+            const uint32_t x0 = (q % P.tiles_x) * kResTile;
+            q /= P.tiles_x;
+            const uint32_t y0 = (q % P.tiles_y) * kResTile + m * kResMRows, img = q / P.tiles_y;
+            const uint32_t px = x0 + (r % kResTile), py = y0 + r / kResTile;
+            const bool inb = px < P.w && py < P.h;
+            const size_t pix = (static_cast<size_t>(img) * P.h + py) * P.w + px;
+            // The staging tile is free once the store before it has read it; the four warps learn here
+            // whether all of them saw the accumulators, so that they leave together.
+            if (r == 0) tma_store_wait_read();
+            if (!bar_sync_and(1u + m, kTileM, mbar_wait(&acc_full[set], (i >> 1) & 1u, P.err))) break;
+            tc_fence_after();
+            for (uint32_t j = 0; j < P.cout / 32u; ++j) {
+                uint32_t v[32];
+                tmem_ld32(tmem + (((warp & 3u) * 32u) << 16) + set * acc_cols + m * P.cout + j * 32u, v);
+                if (j + 1u == P.cout / 32u) {
+                    tc_fence_before();
+                    mbar_arrive(&acc_empty[set]);
+                }
+                uint8_t *region = out_tile + j * (kTileM * 64u);
+#pragma unroll
+                for (uint32_t half = 0; half < 2; ++half) {
+                    const uint32_t c = j * 32u + half * 16u;
+                    uint32_t h[16], pk[8];
+#pragma unroll
+                    for (uint32_t e = 0; e < 16; ++e) h[e] = v[half * 16u + e];
+                    epilogue_pack(P.out_spec, h, bias + c, pix, c, inb, pk);
+                    if (kPool)
+                        epilogue_pool(P.out_spec, pk, lane, kResTile, inb, img, px, py, P.h, P.w, P.cout, c);
+                    *reinterpret_cast<uint4 *>(region + sw64_offset(r, 2u * half)) =
+                        make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                    *reinterpret_cast<uint4 *>(region + sw64_offset(r, 2u * half + 1u)) =
+                        make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                }
+            }
+            fence_proxy_async_smem();
+            bar_sync(1u + m, kTileM);
+            if (r == 0) {
+                for (uint32_t j = 0; j < P.cout / 32u; ++j)
+                    tma_store_4d(&tmy, out_tile + j * (kTileM * 64u), static_cast<int>(j * 32u),
+                                 static_cast<int>(x0), static_cast<int>(y0), static_cast<int>(img));
+                tma_store_commit();
+            }
+        }
+        if (r == 0) tma_store_wait_read();
     }
     tc_fence_before();
     __syncthreads();
@@ -368,6 +566,7 @@ __global__ void __launch_bounds__(128, 1) k_conv_wgrad(WgradParams P) {
     const uint32_t cg = lane & 3u, kk = lane >> 2;
     // `ok` turns false on a wait timeout; the loop leaves only at a barrier, where every thread agrees.
     bool ok = true;
+    const bool issue = warp == 0 && elect_one();
     for (uint32_t kb = 0; kb < P.kblocks; ++kb) {
         const uint32_t s = kb % kWgStages, u = kb / kWgStages;
         if (u > 0 && ok) ok = mbar_wait(&empty[s], (u - 1) & 1u, P.err);
@@ -405,22 +604,20 @@ __global__ void __launch_bounds__(128, 1) k_conv_wgrad(WgradParams P) {
         }
         fence_proxy_async_smem();
         mbar_arrive(&full[s]);
-        if (tid == 0) {
-            if (!mbar_wait(&full[s], u & 1u, P.err)) {
-                ok = false;
-            } else {
+        if (warp == 0) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], u & 1u, P.err));
+            if (ok) {
                 tc_fence_after();
-                const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+                const uint32_t da = smem_desc_sw64(smem_u32(a)), db = smem_desc_sw64(smem_u32(b));
 #pragma unroll
                 for (uint32_t k2 = 0; k2 < 2; ++k2)
-                    mma_bf16(tmem, smem_desc_sw64(sa + 32u * k2), smem_desc_sw64(sb + 32u * k2), idesc,
-                             (kb | k2) != 0u);
-                mma_commit(&empty[s]);
+                    mma_bf16(tmem, da + 2u * k2, kDescHiSw64, db + 2u * k2, kDescHiSw64, idesc, kb | k2, issue);
+                mma_commit(&empty[s], issue);
             }
         }
     }
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) mma_commit(accum);
+    if (warp == 0 && ok) mma_commit(accum, issue);
     bool ready = ok && mbar_wait(accum, 0, P.err);
     ready = __all_sync(0xFFFFFFFFu, ready);
     tc_fence_after();
@@ -536,24 +733,23 @@ __global__ void __launch_bounds__(128, 1)
             for (uint32_t sp = 0; sp < cspans; ++sp)
                 tma_load_4d(b + sp * kWgtSpanBytes, &tmdy, &full[s], static_cast<int>(sp * 32u), x0, y0, img);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         const uint32_t idesc = idesc_bf16(kTileM, P.cout, true, true);
+        const bool issue = elect_one();
         bool ok = true;
         for (uint32_t i = 0; i < nkb; ++i) {
             const uint32_t s = i % nst, u = i / nst;
-            if (!mbar_wait(&full[s], u & 1u, P.err)) {
-                ok = false;
-                break;
-            }
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], u & 1u, P.err));
+            if (!ok) break;
             tc_fence_after();
-            const uint32_t a = smem_u32(smem + s * stage_bytes), b = a + 4u * kWgtSpanBytes;
+            const uint32_t a = smem_desc_mn_sw64(smem_u32(smem + s * stage_bytes), kWgtSpanBytes);
+            const uint32_t b = a + 4u * kWgtSpanBytes / 16u;
 #pragma unroll
             for (uint32_t k16 = 0; k16 < kWgtPix / 16u; ++k16)
-                mma_bf16(tmem, smem_desc_mn_sw64(a + k16 * 1024u, kWgtSpanBytes),
-                         smem_desc_mn_sw64(b + k16 * 1024u, kWgtSpanBytes), idesc, (i | k16) != 0u);
-            mma_commit(&empty[s]);
+                mma_bf16(tmem, a + k16 * 64u, kDescHiSw64, b + k16 * 64u, kDescHiSw64, idesc, i | k16, issue);
+            mma_commit(&empty[s], issue);
         }
-        if (ok && nkb > 0) mma_commit(accum);
+        if (ok && nkb > 0) mma_commit(accum, issue);
     }
     __syncwarp();
 
@@ -672,6 +868,101 @@ OutSpec out_spec(const NhwcView &y, const ConvEpilogue &epi) {
     return o;
 }
 
+// Ring depth and CTAs per SM of a layer: two CTAs while two boxes each still fit, else one with as many boxes
+// as fit, up to six (1920 x 1088, 96 -> 32: 155 us with two CTAs of two boxes, 163 us with one of six; 960 x
+// 544, 32 -> 64: 27 and 35 us; 1920 x 1088, 32 -> 32: 59 us with two CTAs of three boxes, 67 us with three of
+// two). 0 stages when the weights leave no room or the accumulators need more than a CTA's share of TMEM.
+struct ResPlan {
+    uint32_t stages, ctas;
+};
+ResPlan res_plan(uint32_t cin, uint32_t cout) {
+    if (2u * kResM * cout > 256u) return {0, 0};
+    for (uint32_t ctas = kResCtas; ctas > 0; --ctas) {
+        const uint32_t room = std::min<uint32_t>(kMaxDynSmem, 228u * 1024u / ctas - 1024u);
+        const uint32_t fixed = res_smem_bytes(cin, cout, 0);
+        const uint32_t stages = room > fixed ? (room - fixed) / kResBoxBytes : 0u;
+        if (stages >= 2u) return {std::min(stages, kResStages), ctas};
+    }
+    return {0, 0};
+}
+
+unsigned long long res_tiles(const ConvGeom &g) {
+    return static_cast<unsigned long long>((g.w + kResTile - 1) / kResTile) * ((g.h + kResTile - 1) / kResTile) * g.n;
+}
+
+// Layers that fit go to k_conv_res from four tiles per SM on: with fewer, the CTAs pay for their weights and
+// the empty ends of the pipeline over too few tiles (16 x 64 x 64 pixels, 64 -> 64, 1.7 tiles per SM: 10.3 us
+// against 9.8; 640 x 360, 6 tiles: 20.6 against 25.2). Up to 8 columns its 16-column tiles would be half empty.
+bool res_takes(uint32_t cin, uint32_t cout, const ConvGeom &g) {
+    static const int sms = device_sms();
+    const unsigned long long tiles = res_tiles(g);
+    return g.w > 8u && tiles >= 4ull * static_cast<unsigned long long>(sms) && tiles <= 0x7FFFFFFFull &&
+           res_plan(cin, cout).stages != 0;
+}
+
+cudaError_t forward_resident(const NhwcView &x, const void *w, uint32_t cout, const NhwcView &y, const ConvGeom &g,
+                             const ConvEpilogue &epi, uint32_t *err, cudaStream_t stream) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return cudaErrorNotSupported;
+    CUtensorMap tmx, tmw, tmy;
+    {
+        const cuuint64_t dims[4] = {x.channels, g.w, g.h, g.n};
+        const cuuint64_t strides[3] = {static_cast<cuuint64_t>(x.ld) * 2u, static_cast<cuuint64_t>(x.ld) * 2u * g.w,
+                                       static_cast<cuuint64_t>(x.ld) * 2u * g.w * g.h};
+        const cuuint32_t box[4] = {32u, kResTile, kResTile + 2u, 1u};
+        const cuuint32_t es[4] = {1u, 1u, 1u, 1u};
+        if (enc(&tmx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, x.ptr, dims, strides, box, es,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    {
+        const cuuint64_t dims[2] = {9u * x.channels, cout};
+        const cuuint64_t strides[1] = {9u * x.channels * 2u};
+        const cuuint32_t box[2] = {32u, cout};
+        const cuuint32_t es[2] = {1u, 1u};
+        if (enc(&tmw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(w), dims, strides, box, es,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    {
+        const cuuint64_t dims[4] = {cout, g.w, g.h, g.n};
+        const cuuint64_t strides[3] = {static_cast<cuuint64_t>(y.ld) * 2u, static_cast<cuuint64_t>(y.ld) * 2u * g.w,
+                                       static_cast<cuuint64_t>(y.ld) * 2u * g.w * g.h};
+        const cuuint32_t box[4] = {32u, kResTile, kResMRows, 1u};
+        const cuuint32_t es[4] = {1u, 1u, 1u, 1u};
+        if (enc(&tmy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, y.ptr, dims, strides, box, es,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    ResParams P{};
+    P.n = g.n;
+    P.h = g.h;
+    P.w = g.w;
+    P.cin = x.channels;
+    P.cout = cout;
+    P.tiles_x = (g.w + kResTile - 1) / kResTile;
+    P.tiles_y = (g.h + kResTile - 1) / kResTile;
+    P.tiles = static_cast<uint32_t>(res_tiles(g));
+    const ResPlan plan = res_plan(P.cin, cout);
+    P.stages = plan.stages;
+    P.out_spec = out_spec(y, epi);
+    P.err = err;
+    static std::once_flag attr;
+    std::call_once(attr, [] {
+        cudaFuncSetAttribute(k_conv_res<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+        cudaFuncSetAttribute(k_conv_res<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+    });
+    const size_t smem = launch_smem(res_smem_bytes(P.cin, cout, P.stages), tmem_columns(2u * kResM * cout));
+    if (smem == 0) return cudaErrorInvalidConfiguration;
+    const uint32_t grid = std::min(P.tiles, plan.ctas * static_cast<uint32_t>(device_sms()));
+    auto *kern = P.out_spec.pool ? k_conv_res<true> : k_conv_res<false>;
+    kern<<<grid, kResThreads, smem, stream>>>(tmx, tmw, tmy, P);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t conv_wait_probe(uint32_t *err, cudaStream_t stream) {
@@ -688,6 +979,7 @@ cudaError_t conv3x3_forward(const NhwcView &x, const void *w, uint32_t cout, con
     if (epi.mask.ptr && (epi.mask.channels != cout || epi.mask.ld % 8u || !aligned16(epi.mask.ptr)))
         return cudaErrorInvalidValue;
     if (epi.pool && ((g.h | g.w) & 1u || !aligned16(epi.pool))) return cudaErrorInvalidValue;
+    if (res_takes(x.channels, cout, g)) return forward_resident(x, w, cout, y, g, epi, err, stream);
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     // Tiles of 16 x 8 pixels (8 x 16 below 16 columns): a multiple of 8 columns, so that the row taps'

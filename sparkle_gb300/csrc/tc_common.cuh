@@ -125,6 +125,24 @@ __device__ __forceinline__ void tma_prefetch_desc(const void *tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
+// Named barrier `id` over `threads` threads (whole warps), and the same with the AND of a predicate.
+__device__ __forceinline__ void bar_sync(uint32_t id, uint32_t threads) {
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ bool bar_sync_and(uint32_t id, uint32_t threads, bool pred) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"(id), "r"(threads), "r"(pred ? 1u : 0u)
+        : "memory");
+    return r != 0;
+}
+
 // Generic-proxy shared-memory writes made visible to the async proxy (tcgen05.mma reads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -153,22 +171,43 @@ __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// True in one lane of a converged warp, the same lane every time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r));
+    return r != 0;
+}
+
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by the lane with `issue` set. The whole warp calls it with the same
+// operands, outside divergent code: the descriptors, given as (low, high) words, then stay in uniform
+// registers, where the instruction takes them from. Under `lane == 0` each MMA first had its operands moved
+// there one by one (forward 32 -> 32 at 1920 x 1088: 95 us, now 88; 96 -> 32: 184, now 174).
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                         uint32_t idesc, uint32_t accumulate, bool issue) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        ".reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %2};\n\t"
+        "mov.b64 b, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(issue ? 1u : 0u)
         : "memory");
 }
 
-// Arrives once on `bar` when every MMA this thread issued before has completed.
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
+// Arrives once on `bar` when every MMA the issuing lane issued before has completed.
+__device__ __forceinline__ void mma_commit(uint64_t *bar, bool issue) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"(issue ? 1u : 0u)
+        : "memory");
 }
 
 // 32 lanes x 16 consecutive 32-bit columns: thread `lane` of the warp receives row (lane base + lane). The
@@ -184,30 +223,40 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "memory");
 }
 
-// Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row atoms 512 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);      // start address
-    d |= static_cast<uint64_t>(1u) << 16;                      // leading byte offset (unused when swizzled)
-    d |= static_cast<uint64_t>(512u >> 4) << 32;               // stride byte offset
-    d |= static_cast<uint64_t>(1u) << 46;                      // descriptor version
-    d |= static_cast<uint64_t>(4u) << 61;                      // SWIZZLE_64B
-    return d;
+// The same over 32 columns.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
 }
 
-// Shared-memory matrix descriptor of an MN-major operand, 64-byte swizzle: the tile is rows of 64 bytes
-// (32 consecutive BF16 of the M or N dimension), one row per K index; 8 consecutive K rows form a 512-byte
-// swizzle atom (stride byte offset = 512 between 8-row K groups) and 32-element M/N spans sit `span_bytes`
-// apart (leading byte offset). This is the layout a 64-byte-swizzled TMA box {32 channels, pixels} lands
-// in, with K = pixels.
-__device__ __forceinline__ uint64_t smem_desc_mn_sw64(uint32_t saddr, uint32_t span_bytes) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);              // start address
-    d |= static_cast<uint64_t>((span_bytes >> 4) & 0x3FFFu) << 16;   // leading byte offset: next M/N span
-    d |= static_cast<uint64_t>(512u >> 4) << 32;                     // stride byte offset: next 8 K rows
-    d |= static_cast<uint64_t>(1u) << 46;                            // descriptor version
-    d |= static_cast<uint64_t>(4u) << 61;                            // SWIZZLE_64B
-    return d;
+// Shared-memory matrix descriptors as two words. The low word holds the start address and the leading byte
+// offset, both in 16-byte units, so a tile that starts `bytes` further is the low word plus bytes / 16; the
+// high word (stride byte offset, version, swizzle) is the same for all tiles of a layout.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr, uint32_t leading_bytes) {
+    return ((saddr >> 4) & 0x3FFFu) | ((leading_bytes >> 4) & 0x3FFFu) << 16;
+}
+__host__ __device__ constexpr uint32_t smem_desc_hi(uint32_t stride_bytes, uint32_t swizzle) {
+    return ((stride_bytes >> 4) & 0x3FFFu) | (1u << 14) | (swizzle << 29);
+}
+constexpr uint32_t kSwizzle64 = 4;
+
+// K-major, 64-byte swizzle: 8-row atoms 512 bytes apart, leading byte offset unused. MN-major, 64-byte swizzle:
+// the tile is rows of 64 bytes (32 consecutive BF16 of the M or N dimension), one row per K index; 8
+// consecutive K rows form a 512-byte swizzle atom (stride byte offset = 512 between 8-row K groups) and
+// 32-element M/N spans sit `span_bytes` apart (leading byte offset). This is the layout a 64-byte-swizzled TMA
+// box {32 channels, pixels} lands in, with K = pixels.
+constexpr uint32_t kDescHiSw64 = smem_desc_hi(512u, kSwizzle64);
+__device__ __forceinline__ uint32_t smem_desc_sw64(uint32_t saddr) { return smem_desc_lo(saddr, 16u); }
+__device__ __forceinline__ uint32_t smem_desc_mn_sw64(uint32_t saddr, uint32_t span_bytes) {
+    return smem_desc_lo(saddr, span_bytes);
 }
 
 // Instruction descriptor of kind::f16: BF16 A and B, FP32 D, M x N; A and B K-major unless `a_mn` /
