@@ -475,7 +475,9 @@ struct DnRange {
 struct spk_denoiser {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;  // weight gradients, beside the chain of input gradients; idle between calls
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // stream -> side, side -> stream
     std::string error;
     std::vector<Layer> layers;
     size_t nparams = 0, nweights = 0;
@@ -614,12 +616,16 @@ cudaError_t conv_dgrad(spk_denoiser *dn, uint32_t li, const NhwcView &dy, const 
     return conv3x3_forward(dy, dn->wt.p + L.wb_off, L.cin, dx, g, epi, dn->err.p, dn->stream);
 }
 
-// Weight gradient of layer li; its bias gradient goes into `bias` (dy stays in its buffer until the end of backward).
+// Weight gradient of layer li; its bias gradient goes into `bias`. It runs on the side stream from where `stream`
+// stands now: x and dy are complete there, and nothing writes their buffers until backward has joined the streams.
 cudaError_t layer_grads(spk_denoiser *dn, BiasTable &bias, uint32_t li, const NhwcView &x, const NhwcView &dy,
                         const ConvGeom &g) {
     const Layer &L = dn->layers[li];
-    cudaError_t e = conv3x3_wgrad(x, dy, dn->grads.p + L.w_off, g, dn->err.p, dn->stream);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
+    if ((e = cudaEventRecord(dn->ev_fork, dn->stream)) != cudaSuccess ||
+        (e = cudaStreamWaitEvent(dn->side, dn->ev_fork)) != cudaSuccess ||
+        (e = conv3x3_wgrad(x, dy, dn->grads.p + L.w_off, g, dn->err.p, dn->side)) != cudaSuccess)
+        return e;
     const uint32_t k = bias.count++;
     bias.c[k] = dy.channels;
     bias.g[k] = static_cast<const bf16 *>(dy.ptr);
@@ -665,7 +671,12 @@ cudaError_t forward(spk_denoiser *dn, const float *feat, uint32_t n, uint32_t h,
     return cudaGetLastError();
 }
 
-cudaError_t backward(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_t wp) {
+// The chain of input gradients (dn->stream) with each layer's weight gradient beside it (dn->side). Both are short
+// launches that fill few SMs on the coarse levels, and the weight gradients, 0.49 ms of the kernels' time, wait for
+// nothing but their layer's input: gradients of 16 crops of 128 x 128 1333 -> 1077 us.
+// CTAs of both streams may ask for more TMEM than an SM has; the one that comes second then waits in tcgen05.alloc
+// for a CTA that holds its own columns already and waits for none.
+cudaError_t backward_launches(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_t wp) {
     cudaError_t e;
     auto G = [&](uint32_t l) { return ConvGeom{n, hp >> l, wp >> l}; };
     BiasTable bias{};
@@ -715,6 +726,14 @@ cudaError_t backward(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_t wp) {
     }
     k_bias_grads<<<bias.first[bias.count], 256, 0, dn->stream>>>(bias);
     return cudaGetLastError();
+}
+
+// All of backward, on dn->stream for the caller. The streams are joined after a failure too.
+cudaError_t backward(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_t wp) {
+    const cudaError_t e = backward_launches(dn, n, hp, wp);
+    cudaError_t j = cudaEventRecord(dn->ev_join, dn->side);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(dn->stream, dn->ev_join);
+    return e != cudaSuccess ? e : j;
 }
 
 spk_status check_errors(spk_denoiser *dn) {
@@ -768,6 +787,9 @@ spk_status spk_dn_create(int32_t device, uint64_t seed, spk_denoiser **out) {
     cudaError_t e;
     if ((e = cudaSetDevice(device)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&dn->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&dn->side, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&dn->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&dn->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreate(&dn->ev0)) != cudaSuccess || (e = cudaEventCreate(&dn->ev1)) != cudaSuccess ||
         (e = dn->params.ensure(dn->nparams)) != cudaSuccess || (e = dn->grads.ensure(dn->nparams)) != cudaSuccess ||
         (e = dn->adam_m.ensure(dn->nparams)) != cudaSuccess || (e = dn->adam_v.ensure(dn->nparams)) != cudaSuccess ||
@@ -789,6 +811,7 @@ spk_status spk_dn_destroy(spk_denoiser *dn) {
     if (!dn) return SPK_OK;
     cudaSetDevice(dn->device);
     if (dn->stream) cudaStreamSynchronize(dn->stream);
+    if (dn->side) cudaStreamSynchronize(dn->side);
     DBuf<float> *fb[] = {&dn->params, &dn->grads, &dn->adam_m, &dn->adam_v, &dn->frame};
     for (auto *b : fb) b->release();
     DBuf<bf16> *bb[] = {&dn->wb, &dn->wt, &dn->x0, &dn->out, &dn->gout, &dn->eb4, &dn->conv_wt_scratch};
@@ -807,6 +830,9 @@ spk_status spk_dn_destroy(spk_denoiser *dn) {
     dn->loss.release();
     if (dn->ev0) cudaEventDestroy(dn->ev0);
     if (dn->ev1) cudaEventDestroy(dn->ev1);
+    if (dn->ev_fork) cudaEventDestroy(dn->ev_fork);
+    if (dn->ev_join) cudaEventDestroy(dn->ev_join);
+    if (dn->side) cudaStreamDestroy(dn->side);
     if (dn->stream) cudaStreamDestroy(dn->stream);
     delete dn;
     return SPK_OK;
