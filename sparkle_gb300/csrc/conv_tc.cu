@@ -6,7 +6,7 @@
 //                  input box {32 ch, tw px, mt * th + 2 rows, 1 image} shifted by dx and reaching one row
 //                  above and below the tile (zero fill outside the image = the conv's padding), and three
 //                  2-D loads of the weight slices {32, cout} of the taps (dy, dx), dy = -1, 0, 1, into a
-//                  ring of 2-4 stages;
+//                  ring of 2-6 stages;
 //   warp 1         MMA issuer: per stage, row tap dy and M tile m, two kind::f16 MMAs (K = 16 each) whose A
 //                  operand starts (m * th + dy + 1) * tw rows into the input box -- a whole number of 8-row
 //                  swizzle atoms, so one box serves all three row taps of all M tiles and one weight slice
@@ -35,9 +35,10 @@ namespace {
 using namespace tc;
 
 constexpr uint32_t kTileM = 128;
-constexpr uint32_t kStages = 4;
+constexpr uint32_t kStages = 6;
 constexpr uint32_t kATileBytes = kTileM * 64;  // 128 rows x 32 bf16
 constexpr uint32_t kMaxCout = 256;
+constexpr uint32_t kFwdExtra = 1024 + 256;  // forward CTA's shared memory beside the ring: alignment, barriers
 #ifndef SPK_CONV_STAGE_BUDGET_KB
 #define SPK_CONV_STAGE_BUDGET_KB 32  // shared memory for the forward kernel's ring (KB): 2 stages, more CTAs per SM
 #endif
@@ -856,6 +857,22 @@ uint32_t conv_mtiles(const ConvGeom &g, uint32_t tw, uint32_t th, uint32_t cout)
     return 1;
 }
 
+// Ring depth of a forward layer of `nk` K blocks and `tiles` CTAs, at least 2. A large grid takes the stage
+// budget: a small ring leaves room for more CTAs per SM, whose loads cover each other. A grid of one wave leaves
+// shared memory idle, and a CTA waits for a load every second K block: there the ring takes what the CTAs of one
+// SM leave, up to 6 stages. Inference of 256 x 256 280 -> 262 us, of 640 x 360 361 -> 340, gradients of 4 crops of
+// 128 x 96 683 -> 638; of a full-HD image, whose coarse levels alone change, 1121 -> 1114.
+uint32_t fwd_stages(uint32_t stage_bytes, uint32_t nk, unsigned long long tiles, uint32_t tmem_cols) {
+    static const unsigned long long sms = static_cast<unsigned long long>(device_sms());
+    uint32_t stages = (kStageBudget * 1024u) / stage_bytes;
+    const unsigned long long ctas = (tiles + sms - 1) / sms;  // per SM
+    if (ctas <= 512u / tmem_cols) {
+        const size_t room = std::min<size_t>(kMaxDynSmem, 228u * 1024u / static_cast<size_t>(ctas) - 1024u);
+        if (room > kFwdExtra) stages = std::max(stages, static_cast<uint32_t>((room - kFwdExtra) / stage_bytes));
+    }
+    return std::max(2u, std::min({kStages, nk, stages}));
+}
+
 OutSpec out_spec(const NhwcView &y, const ConvEpilogue &epi) {
     OutSpec o{};
     o.out = static_cast<__nv_bfloat16 *>(y.ptr);
@@ -1035,9 +1052,9 @@ cudaError_t conv3x3_forward(const NhwcView &x, const void *w, uint32_t cout, con
     P.tiles_y = (g.h + rows - 1) / rows;
     P.a_bytes = fwd_a_bytes(tw, rows);
     P.stage_bytes = fwd_stage_bytes(tw, rows, cout);
-    // Ring depth: up to 4 stages within the stage budget, never more than the K blocks of a tile (3 per 32
-    // channels). A smaller ring leaves room for more CTAs per SM.
-    P.stages = std::max(2u, std::min({kStages, 3u * (x.channels / 32u), (kStageBudget * 1024u) / P.stage_bytes}));
+    const unsigned long long tiles = static_cast<unsigned long long>(P.tiles_x) * P.tiles_y * g.n;
+    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;
+    P.stages = fwd_stages(P.stage_bytes, 3u * (x.channels / 32u), tiles, tmem_columns(mt * cout));
     P.out_spec = out_spec(y, epi);
     // The staged tile (mt x 128 pixels x cout BF16) must fit in the ring it reuses.
     P.stage_out = (SPK_CONV_TMA_STORE && kTileM * 2u * mt * cout <= P.stages * P.stage_bytes) ? 1u : 0u;
@@ -1047,9 +1064,7 @@ cudaError_t conv3x3_forward(const NhwcView &x, const void *w, uint32_t cout, con
         cudaFuncSetAttribute(k_conv_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
         cudaFuncSetAttribute(k_conv_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
     });
-    const unsigned long long tiles = static_cast<unsigned long long>(P.tiles_x) * P.tiles_y * g.n;
-    if (tiles > 0x7FFFFFFFull) return cudaErrorInvalidValue;
-    const size_t smem = launch_smem(P.stages * P.stage_bytes + 1024 + 256, tmem_columns(mt * cout));
+    const size_t smem = launch_smem(P.stages * P.stage_bytes + kFwdExtra, tmem_columns(mt * cout));
     if (smem == 0) return cudaErrorInvalidConfiguration;
     auto *kern = P.out_spec.pool ? k_conv_fwd<true> : k_conv_fwd<false>;
     kern<<<static_cast<unsigned>(tiles), kFwdThreads, smem, stream>>>(tmx, tmw, tmy, P);

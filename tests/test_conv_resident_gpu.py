@@ -55,3 +55,20 @@ def test_network_batch_matches_single_images(dn, h, w):
     batch = dn.infer(feats).clone()
     for i in range(n):
         assert torch.equal(batch[i], dn.infer(feats[i:i + 1].contiguous())[0])
+
+
+@pytest.mark.parametrize("cin,cout", [(32, 96), (128, 128), (224, 96), (32, 256)])
+@pytest.mark.parametrize("waves,extra", [(1, 0), (1, 1), (2, 0), (2, 1)])
+def test_ring_depths_agree(dn, cin, cout, waves, extra):
+    """Wide layers on grids of one and two CTAs per SM and just above: the ring's depth changes there, the sums
+    do not. One tile of 16 x 8 pixels per image."""
+    n = waves * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    gen = torch.Generator(device="cuda").manual_seed(cin + cout + n)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=gen).to(torch.bfloat16)
+    x, wt, bias = rand(n, 8, 16, cin), rand(cout, 9, cin) * 0.1, torch.randn(cout, device="cuda", generator=gen)
+    y = torch.zeros(n, 8, 16, cout, device="cuda", dtype=torch.bfloat16)
+    one = y.clone()
+    dn.conv3x3(0, x, cin, wt, y, cout, n, 8, 16, bias=bias, relu=True)
+    for i in (0, 1, n // 2, n - 1):
+        dn.conv3x3(0, x[i:], cin, wt, one[i:], cout, 1, 8, 16, bias=bias, relu=True)
+        assert torch.equal(y[i], one[i])
