@@ -43,9 +43,9 @@ struct BlasRefit {
 // MeshRenderProxy.cpp:80-86) from the new positions.
 cudaError_t launch_refit_triangles(const BlasRefit &r, cudaStream_t stream);
 
-// Refits the nodes root + [first, last): one depth of the breadth-first node order the builders emit,
-// launched deepest depth first so that every inner child is refitted before its parent.
-cudaError_t launch_refit_nodes(const BlasRefit &r, uint32_t first, uint32_t last, cudaStream_t stream);
+// Refits the BLAS's nodes and their boxes in r.boxes, deepest depth first. `levels` [count + 1]: the first node
+// of each depth of the breadth-first order the builders emit, levels[0] = 0, then the node count.
+cudaError_t launch_refit_nodes(const BlasRefit &r, const uint32_t *levels, uint32_t count, cudaStream_t stream);
 
 // Writes new normals (and, when given, tangents xyzw) into the vertex records verts[3*(vert_base + v)].
 cudaError_t launch_update_vertices(float4 *verts, uint32_t vert_base, uint32_t num_vertices, const float *normals,

@@ -1198,6 +1198,7 @@ spk_status spk_update_mesh(spk_ctx *ctx, uint32_t mesh_id, uint32_t num_vertices
             (e = launch_update_vertices(ctx->verts.ptr, b.vert_base, num_vertices, dn, dt, ctx->stream)) != cudaSuccess)
             return cuda_fail(ctx, e, "vertex attributes");
     }
+    float box[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // the refitted root's
     if (b.root != kInvalid) {
         if (ctx->dyn_boxes.count < 6ull * b.node_count && (e = alloc(ctx->dyn_boxes, 6ull * b.node_count)) != cudaSuccess)
             return cuda_fail(ctx, e, "refit scratch");
@@ -1213,22 +1214,32 @@ spk_status spk_update_mesh(spk_ctx *ctx, uint32_t mesh_id, uint32_t num_vertices
         r.tri_count = b.tri_count;
         r.num_faces = num_faces;
         r.num_vertices = num_vertices;
-        if ((e = launch_refit_triangles(r, ctx->stream)) != cudaSuccess) return cuda_fail(ctx, e, "refit");
-        for (size_t l = b.levels.size() - 1; l-- > 0;)
-            if ((e = launch_refit_nodes(r, b.levels[l], b.levels[l + 1], ctx->stream)) != cudaSuccess)
-                return cuda_fail(ctx, e, "refit");
+        if ((e = launch_refit_triangles(r, ctx->stream)) != cudaSuccess ||
+            (e = launch_refit_nodes(r, b.levels.data(), static_cast<uint32_t>(b.levels.size() - 1), ctx->stream)) !=
+                cudaSuccess ||
+            (e = cudaMemcpyAsync(box, r.boxes, sizeof(box), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+            return cuda_fail(ctx, e, "refit");
     }
-    // The mesh's local box over its faces' vertices, as the BLAS build takes it.
+    // The mesh's local box over its faces' vertices, as the BLAS build takes it: the refitted root's box, which
+    // holds the same minima and maxima when the tree holds every face. Where a bound may be the refit's start
+    // value or is not finite the host walks the faces (2.1M of them: 13 ms, which every update took before).
     MeshBlas &mb = dy.blas[mesh_id];
-    for (int a = 0; a < 3; ++a) {
-        mb.bounds[a] = std::numeric_limits<double>::max();
-        mb.bounds[3 + a] = -std::numeric_limits<double>::max();
-    }
-    for (uint32_t i : dy.indices[mesh_id])
+    bool root_box = b.root != kInvalid && b.tri_count == num_faces;
+    for (float v : box) root_box = root_box && std::fabs(v) < std::numeric_limits<float>::max();
+    if (root_box) {
+        std::copy(box, box + 6, mb.bounds);
+    } else {
         for (int a = 0; a < 3; ++a) {
-            mb.bounds[a] = std::min(mb.bounds[a], static_cast<double>(pos[3ull * i + a]));
-            mb.bounds[3 + a] = std::max(mb.bounds[3 + a], static_cast<double>(pos[3ull * i + a]));
+            mb.bounds[a] = std::numeric_limits<double>::max();
+            mb.bounds[3 + a] = -std::numeric_limits<double>::max();
         }
+        for (uint32_t i : dy.indices[mesh_id])
+            for (int a = 0; a < 3; ++a) {
+                mb.bounds[a] = std::min(mb.bounds[a], static_cast<double>(pos[3ull * i + a]));
+                mb.bounds[3 + a] = std::max(mb.bounds[3 + a], static_cast<double>(pos[3ull * i + a]));
+            }
+    }
     st = rebuild_top(ctx);
     if (st != SPK_OK) return st;
     if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cuda_fail(ctx, e, "refit");

@@ -224,3 +224,32 @@ def test_empty_instance_list_and_back(ctx, cornell):
     ctx.set_scene(sc)
     ctx.update_mesh(len(scene.meshes), np.ones((3, 3), np.float32))
     assert np.array_equal(render(ctx, (sc, cam_args), cfg).view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("side,scale,offset", [
+    (1, (1.0, 1.0, 1.0), (0.0, 0.0, 0.0)),              # two triangles, one node
+    (5, (255.0, 1.0, 1e-20), (-1e-20, 0.0, 0.0)),       # extents that need more than a double to hold
+    (40, (1.0, 1.0, 0.0), (1e6, -1e6, 3.0)),            # flat and far from the origin: few distinct coordinates
+    (40, (1e-30, 1e25, 1e-3), (0.0, 0.0, 1e5)),         # beyond the range of the float path
+    (120, (7.0, 3.0, 0.7), (0.1, -2.0, 100.0)),         # depths of more and of fewer than 512 nodes
+    (120, (1020.0, 510.0, 255.0), (0.0, 0.0, -255.0)),  # extents and boxes on the grid
+])
+def test_identity_refit_ranges(ctx, side, scale, offset):
+    """A refit with unchanged positions reproduces the host builder's nodes byte for byte."""
+    rng = np.random.default_rng(side)
+    x, y = np.meshgrid(np.arange(side + 1) / side, np.arange(side + 1) / side, indexing="ij")
+    pos = np.stack([x, y, np.round(rng.random(x.shape) * 8) / 8], -1).reshape(-1, 3)
+    pos = (pos * np.array(scale) + np.array(offset)).astype(np.float32)
+    a = (np.arange(side)[:, None] * (side + 1) + np.arange(side)[None, :]).reshape(-1)
+    faces = np.concatenate([np.stack([a, a + side + 1, a + 1], 1), np.stack([a + 1, a + side + 1, a + side + 2], 1)])
+    scene, _ = copy.deepcopy(scenes.cornell_box(0))
+    mesh = scene.meshes[0]
+    mesh.positions = pos
+    mesh.normals = np.tile(np.float32([0, 0, 1]), (len(pos), 1))
+    mesh.tangents = None
+    mesh.uvs = None
+    mesh.indices = faces.astype(np.uint32)
+    ctx.set_scene(scene)
+    before = ctx.bvh_nodes()
+    ctx.update_mesh(0, pos)
+    assert np.array_equal(before, ctx.bvh_nodes())
