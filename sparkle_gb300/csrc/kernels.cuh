@@ -32,6 +32,7 @@ struct Counters {
     unsigned long long node_visits;
     unsigned long long tri_tests;
     unsigned long long queue_counters[12];
+    unsigned long long walk_start, walk_ns;  // wavefront: the extend stage that runs, and the time of those before it
     unsigned int seed_base, seed_step;  // multi-frame pass: frame k's samples are seeded with seed_base + k * seed_step
 };
 
@@ -48,18 +49,12 @@ struct LaunchEvents {
     cudaEvent_t *pairs = nullptr;  // 2 * capacity events
     int capacity = 0;
     int used = 0;
-    float graph_ms = 0.f;   // traversal time measured inside replayed CUDA graphs
-    int graph_launches = 0;  // traversal launches inside replayed CUDA graphs
-    cudaEvent_t *graph_pairs = nullptr;  // events of a replay whose times are still to be read (after the stream is done)
-    int graph_pending = 0;
-    // cudaEventRecordExternal while a stream is captured: the record becomes a graph node that every replay
-    // performs (a plain record under capture only orders work inside the graph).
-    unsigned record_flags = cudaEventRecordDefault;
+    int graph_launches = 0;  // traversal launches inside replayed CUDA graphs: their time is in Counters::walk_ns
     void before(cudaStream_t s) {
-        if (pairs && used < capacity) cudaEventRecordWithFlags(pairs[2 * used], s, record_flags);
+        if (pairs && used < capacity) cudaEventRecord(pairs[2 * used], s);
     }
     void after(cudaStream_t s) {
-        if (pairs && used < capacity) cudaEventRecordWithFlags(pairs[2 * used++ + 1], s, record_flags);
+        if (pairs && used < capacity) cudaEventRecord(pairs[2 * used++ + 1], s);
     }
 };
 

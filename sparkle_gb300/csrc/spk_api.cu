@@ -341,9 +341,7 @@ cudaError_t prepare_events(spk_ctx *ctx, size_t pairs) {
     ctx->launch_events.pairs = ctx->event_pool.data();
     ctx->launch_events.capacity = static_cast<int>(ctx->event_pool.size() / 2);
     ctx->launch_events.used = 0;
-    ctx->launch_events.graph_ms = 0.f;
     ctx->launch_events.graph_launches = 0;
-    ctx->launch_events.graph_pending = 0;
     return cudaSuccess;
 }
 
@@ -1964,18 +1962,12 @@ spk_status spk_get_stats(spk_ctx *ctx, spk_stats *out) {
         ctx->last.device_ms = ms;
         float tms = 0.f;
         LaunchEvents &le = ctx->launch_events;
-        for (int k = 0; k < le.graph_pending; ++k) {
-            float x = 0.f;
-            cudaEventElapsedTime(&x, le.graph_pairs[2 * k], le.graph_pairs[2 * k + 1]);
-            le.graph_ms += x;
-        }
-        le.graph_pending = 0;
         for (int k = 0; k < le.used; ++k) {
             float x = 0.f;
             cudaEventElapsedTime(&x, le.pairs[2 * k], le.pairs[2 * k + 1]);
             tms += x;
         }
-        ctx->last.trace_kernel_ms = tms + le.graph_ms;
+        ctx->last.trace_kernel_ms = tms + (le.graph_launches > 0 ? static_cast<float>(1e-6 * static_cast<double>(c.walk_ns)) : 0.f);
         ctx->last.trace_launches = static_cast<uint32_t>(le.used + le.graph_launches);
         ctx->last.kernel_launches = ctx->launches_in_call;
         ctx->stats_pending = false;

@@ -32,6 +32,40 @@ constexpr int kPacketQueue = 8;
 constexpr int kPacket2Queue = 9;
 constexpr int kNextItem = 10;  // next (frame, pixel) sample item to hand out
 
+// First statement of every kernel that launch_chained starts: from here on the kernel before is complete and its
+// writes are visible.
+__device__ __forceinline__ void after_previous_kernel() { cudaGridDependencySynchronize(); }
+
+// Lets the kernel after this one be launched: its blocks take the places of those that leave and wait in
+// after_previous_kernel. A walk's grid fills the SMs and spreads evenly however it comes in; the shading grids do
+// not, and shading many paths from uneven places costs more than the launch, so a walk of more than kEarlyRays rays
+// lets them in as its last blocks leave (1080p, 64 samples: 101.07 ms with all let in early, 100.63 so, 100.78 with
+// plain launches; 335 x 202, 1 sample: 494, 492 and 552 us with an event node on each side of the walks).
+__device__ __forceinline__ void let_next_kernel_in() { cudaTriggerProgrammaticLaunchCompletion(); }
+constexpr unsigned long long kEarlyRays = 1ull << 20;
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Starts a kernel of the extend / shade loop (128 threads a block) without waiting for the launch latency and the last
+// block of the kernel before it.
+template <class... Params, class... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, cudaStream_t stream, const Args &...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cudaLaunchAttribute chained{};
+    chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    chained.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &chained;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 template <int kKind>
 __device__ __forceinline__ void load_rng(const uint4 *rng, uint32_t pid, Rng &r) {
     const uint4 a = rng[2 * static_cast<size_t>(pid)];
@@ -251,6 +285,7 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
                                                        : SPK_WALK_MIN_BLOCKS)
     k_wf_extend(const __grid_constant__ DevScene S, const __grid_constant__ WavefrontState s, int in_queue,
                 Counters *counters) {
+    after_previous_kernel();
     // The stage's own resets, in place of memset nodes between the kernels: the queues the shade stage fills (nothing
     // reads them now). The shade stage zeroes the walks' cursors in turn.
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -258,12 +293,14 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
         counters->queue_counters[kShadowLen] = 0u;
         counters->queue_counters[kNeeLen] = 0u;
         counters->queue_counters[kShadowCursor] = 0u;
+        if (counters->walk_start == 0u) counters->walk_start = global_ns();  // the stage's first form
     }
     const unsigned long long len = counters->queue_counters[in_queue];
     const unsigned long long p1 = min(counters->queue_counters[kPacketQueue], len);
     const unsigned long long p2 = min(counters->queue_counters[kPacket2Queue], p1);
     const unsigned long long first = kPackets == 2 ? 0ull : kPackets == 1 ? p2 : p1;
     const unsigned long long n = (kPackets == 2 ? p2 : kPackets == 1 ? p1 : len) - first;
+    if (n <= kEarlyRays) let_next_kernel_in();
     if (n == 0) return;
     uint32_t err = 0;
     TraceCounts tc;
@@ -320,9 +357,18 @@ __device__ __forceinline__ uint32_t hits_first(const WavefrontState &s, uint32_t
     return pid;
 }
 
+// The kernel after an extend stage ends its time, so that no event node stands between the two.
+__device__ __forceinline__ void end_walk_time(Counters *counters) {
+    const unsigned long long start = counters->walk_start;
+    if (start == 0u) return;
+    counters->walk_ns += global_ns() - start;
+    counters->walk_start = 0u;
+}
+
 // After an extend stage: its cursors back to zero, and no packet prefix (the next queue is mixed).
 __device__ __forceinline__ void reset_walk(Counters *counters) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        end_walk_time(counters);
         counters->queue_counters[kCursor] = 0u;
         counters->queue_counters[kPacketCursor] = 0u;
         counters->queue_counters[kPacket2Cursor] = 0u;
@@ -334,6 +380,8 @@ __device__ __forceinline__ void reset_walk(Counters *counters) {
 template <int kKind, int kNee>
 __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_wf_shade(DevScene S, FrameBuffers fb, RenderParams p, WavefrontState s,
                                                   int in_queue, uint32_t bounce, Counters *counters) {
+    after_previous_kernel();
+    let_next_kernel_in();
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
@@ -447,6 +495,8 @@ template <int kKind, int kNee>
 __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_mf_shade(DevScene S, DevCamera cam, FrameBuffers fb, RenderParams p,
                                                   WavefrontState s, int in_queue, uint32_t frame_base,
                                                   uint32_t total_items, int common_bounce, Counters *counters) {
+    after_previous_kernel();
+    let_next_kernel_in();
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
@@ -538,6 +588,7 @@ template <int kKey>
 __global__ void __launch_bounds__(256) k_sort_hist(DevScene S, WavefrontState s, int in_queue, Counters *counters) {
     constexpr uint32_t B = SortKey<kKey>::kBuckets;
     __shared__ uint32_t h[B];
+    if (kKey == 0 && blockIdx.x == 0 && threadIdx.x == 0) end_walk_time(counters);
     for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) h[b] = 0;
     __syncthreads();
     const unsigned long long n = counters->queue_counters[in_queue];
@@ -752,6 +803,8 @@ __global__ void __launch_bounds__(128) k_b_generate(DevScene S, BatchParams b, W
 template <int kKind, int kNee>
 __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_b_shade(DevScene S, BatchParams b, WavefrontState s, int in_queue,
                                                  Counters *counters) {
+    after_previous_kernel();
+    let_next_kernel_in();
     uint32_t shadow = 0, err = 0;
     const unsigned long long n = counters->queue_counters[in_queue];
     const int out_queue = in_queue ^ 1;
@@ -807,8 +860,10 @@ template <bool kBatch>
 __global__ void __launch_bounds__(128, SPK_SHADOW_MIN_BLOCKS) k_wf_shadow(const __grid_constant__ DevScene S,
                                                                        const __grid_constant__ WavefrontState s,
                                                                        Counters *counters) {
+    after_previous_kernel();
     uint32_t err = 0;
     const unsigned long long n = counters->queue_counters[kShadowLen];
+    if (n <= kEarlyRays) let_next_kernel_in();
     walk_rays<kTraceOcclusion, false>(
         S, &counters->queue_counters[kShadowCursor], n, kFltMax, err, nullptr,
         [&S, &s](unsigned long long q, f3 &o, f3 &d, float &tmax) {
@@ -834,6 +889,8 @@ __global__ void __launch_bounds__(128, SPK_SHADE_MIN_BLOCKS) k_nee_accumulate(De
                                                                             DevScene S, BatchParams b, WavefrontState s,
                                                                             int out_queue, uint32_t frame_base,
                                                                             uint32_t total_items, Counters *counters) {
+    after_previous_kernel();
+    let_next_kernel_in();
     const unsigned long long n = counters->queue_counters[kNeeLen];
     const uint32_t lane = threadIdx.x & 31u;
     for (unsigned long long q0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x; q0 < n;
@@ -960,27 +1017,22 @@ uint32_t pass_packet_forms(uint32_t frames, const WfTuning &tuning) {
 
 cudaError_t launch_extend(const DevScene &scene, const WavefrontState &s, int in, bool count, Counters *counters,
                           unsigned grid, cudaStream_t stream, LaunchEvents *ev, bool batch, uint32_t packet_forms) {
+    auto launch = [&](auto *kernel) { return launch_chained(kernel, grid, stream, scene, s, in, counters); };
+    cudaError_t e = cudaSuccess;
     if (ev) ev->before(stream);
     if (batch) {
-        if (packet_forms & 2u)
-            (count ? k_wf_extend<true, true, 2> : k_wf_extend<false, true, 2>)<<<grid, 128, 0, stream>>>(scene, s, in,
-                                                                                                         counters);
-        if (packet_forms & 1u)
-            (count ? k_wf_extend<true, true, 1> : k_wf_extend<false, true, 1>)<<<grid, 128, 0, stream>>>(scene, s, in,
-                                                                                                         counters);
-        (count ? k_wf_extend<true, true> : k_wf_extend<false, true>)<<<grid, 128, 0, stream>>>(scene, s, in, counters);
+        if (packet_forms & 2u) e = launch(count ? k_wf_extend<true, true, 2> : k_wf_extend<false, true, 2>);
+        if (e == cudaSuccess && (packet_forms & 1u))
+            e = launch(count ? k_wf_extend<true, true, 1> : k_wf_extend<false, true, 1>);
+        if (e == cudaSuccess) e = launch(count ? k_wf_extend<true, true> : k_wf_extend<false, true>);
     } else {
-        if (packet_forms & 2u)
-            (count ? k_wf_extend<true, false, 2> : k_wf_extend<false, false, 2>)<<<grid, 128, 0, stream>>>(
-                scene, s, in, counters);
-        if (packet_forms & 1u)
-            (count ? k_wf_extend<true, false, 1> : k_wf_extend<false, false, 1>)<<<grid, 128, 0, stream>>>(
-                scene, s, in, counters);
-        (count ? k_wf_extend<true, false> : k_wf_extend<false, false>)<<<grid, 128, 0, stream>>>(scene, s, in,
-                                                                                                 counters);
+        if (packet_forms & 2u) e = launch(count ? k_wf_extend<true, false, 2> : k_wf_extend<false, false, 2>);
+        if (e == cudaSuccess && (packet_forms & 1u))
+            e = launch(count ? k_wf_extend<true, false, 1> : k_wf_extend<false, false, 1>);
+        if (e == cudaSuccess) e = launch(count ? k_wf_extend<true, false> : k_wf_extend<false, false>);
     }
     if (ev) ev->after(stream);
-    return cudaSuccess;
+    return e;
 }
 
 int nee_mode(uint32_t enable_nee, const WfTuning &tuning) {
@@ -1013,9 +1065,9 @@ void enqueue_shadow_stage(const DevScene &scene, const DevCamera &cam, const Fra
                           const BatchParams &b, const WavefrontState &s, uint32_t rng, int out_queue,
                           uint32_t frame_base, uint32_t total_items, Counters *counters, unsigned walk_grid,
                           unsigned shade_grid, cudaStream_t stream) {
-    k_wf_shadow<kMode == 2><<<walk_grid, 128, 0, stream>>>(scene, s, counters);
+    launch_chained(k_wf_shadow<kMode == 2>, walk_grid, stream, scene, s, counters);
     auto *acc = rng == 0 ? k_nee_accumulate<0, kMode> : k_nee_accumulate<1, kMode>;
-    acc<<<shade_grid, 128, 0, stream>>>(cam, fbuf, p, scene, b, s, out_queue, frame_base, total_items, counters);
+    launch_chained(acc, shade_grid, stream, cam, fbuf, p, scene, b, s, out_queue, frame_base, total_items, counters);
 }
 
 }  // namespace
@@ -1081,8 +1133,6 @@ void wavefront_free(WavefrontState &s) {
 
 void chunk_graph_free(ChunkGraph &g) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
-    for (cudaEvent_t ev : g.events)
-        if (ev) cudaEventDestroy(ev);
     const bool enabled = g.enabled;
     g = ChunkGraph{};
     g.enabled = enabled;
@@ -1127,7 +1177,7 @@ cudaError_t launch_render_wavefront(const DevScene &scene, const DevCamera &cam,
             ss = enqueue_material_sort(scene, se, in, counters, num_sms, stream);
             nl += 3;
         }
-        shade<<<shade_blocks, 128, 0, stream>>>(scene, fbuf, p, ss, in, b, counters);
+        launch_chained(shade, shade_blocks, stream, scene, fbuf, p, ss, in, b, counters);
         ++nl;
         if (nee == kNeeDeferred) {
             enqueue_shadow_stage<0>(scene, cam, fbuf, p, BatchParams{}, ss, p.rng, out, 0u, 0u, counters, shadow_grid,
@@ -1213,8 +1263,8 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                     return ce;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                shade<<<shade_blocks, 128, 0, stream>>>(
-                    scene, cam, fbuf, p, ss, in, f0, total_items, together ? static_cast<int>(c) : -1, counters);
+                launch_chained(shade, shade_blocks, stream, scene, cam, fbuf, p, ss, in, f0, total_items,
+                               together ? static_cast<int>(c) : -1, counters);
                 if (nee == kNeeDeferred)
                     enqueue_shadow_stage<1>(scene, cam, fbuf, p, BatchParams{}, ss, p.rng, out, f0, total_items,
                                             counters, shadow_grid, shade_blocks, stream);
@@ -1222,7 +1272,6 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
             return cudaGetLastError();
         };
         bool use_graph = false;
-        LaunchEvents graph_ev{};
         if (graph && graph->enabled) {
             // The graph is keyed by every value its launches take; a new key re-captures it and updates
             // the executable graph in place when the topology allows.
@@ -1258,19 +1307,12 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
             key.iters = iters;
             key.together = together ? 1u : 0u;
             const auto *kb = reinterpret_cast<const unsigned char *>(&key);
-            graph_ev.pairs = graph->events;
-            graph_ev.capacity = static_cast<int>(kChunk);
-            graph_ev.record_flags = cudaEventRecordExternal;
-            if (!graph->events[0]) {
-                for (cudaEvent_t &g_ev : graph->events)
-                    if ((e = cudaEventCreate(&g_ev)) != cudaSuccess) return e;
-            }
             use_graph = true;
             if (!graph->exec || graph->key.size() != sizeof(key) || std::memcmp(graph->key.data(), kb, sizeof(key))) {
                 cudaGraph_t g = nullptr;
                 t_site = "graph capture";
                 if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
-                const cudaError_t enq = enqueue_chunk(ev ? &graph_ev : nullptr);
+                const cudaError_t enq = enqueue_chunk(nullptr);
                 if ((e = cudaStreamEndCapture(stream, &g)) != cudaSuccess) return e;
                 if (enq != cudaSuccess) {
                     cudaGraphDestroy(g);
@@ -1294,12 +1336,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                     return e;
                 }
                 graph->key.assign(kb, kb + sizeof(key));
-                graph->timed = ev != nullptr;
                 ++graph->captures;
-            }
-            if (graph->timed != (ev != nullptr)) {
-                graph->key.clear();  // timing events differ: force a re-capture next time
-                use_graph = false;
             }
         }
         // Each iteration advances every live slot by one segment and no item is started twice, so the
@@ -1311,6 +1348,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
             if (use_graph) {
                 if ((e = cudaGraphLaunch(graph->exec, stream)) != cudaSuccess) return e;
                 ++graph->replays;
+                if (ev) ev->graph_launches += static_cast<int>(iters);
             } else if ((e = enqueue_chunk(ev)) != cudaSuccess) {
                 return e;
             }
@@ -1319,28 +1357,11 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                    (nee == kNeeDeferred ? 2u : 0u)) * iters +
                   extend_launches(packet_forms) - 1u;
             const bool over = at_once && iter >= p.bounce;
-            if (over && iter == iters && num_frames <= kFramesPerPass) {
-                if (use_graph && ev) {
-                    ev->graph_pairs = graph->events;
-                    ev->graph_pending = static_cast<int>(iters);
-                    ev->graph_launches = static_cast<int>(iters);
-                }
-                break;
-            }
+            if (over && iter == iters && num_frames <= kFramesPerPass) break;
             if ((e = cudaMemcpyAsync(s.host_len, qc, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream)) !=
                 cudaSuccess)
                 return e;
             if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
-            t_site = "graph timing events";
-            if (use_graph && ev) {
-                for (uint32_t c = 0; c < iters; ++c) {
-                    float x = 0.f;
-                    if ((e = cudaEventElapsedTime(&x, graph->events[2 * c], graph->events[2 * c + 1])) != cudaSuccess)
-                        return e;
-                    ev->graph_ms += x;
-                }
-                ev->graph_launches += static_cast<int>(iters);
-            }
             if (over || *s.host_len == 0) break;  // (not over: a full chunk, whose last iteration fills queue 0)
             if (iter > max_iters) return cudaErrorLaunchFailure;  // cannot happen: every slot makes progress
         }
@@ -1398,14 +1419,14 @@ cudaError_t launch_render_batch(const DevScene &scene, const BatchParams &b, con
         for (;;) {
             for (uint32_t c = 0; c < kChunk; ++c) {
                 const int in = static_cast<int>(c & 1u), out = in ^ 1;
-                        const WavefrontState se =
+                const WavefrontState se =
                     tuning.ray_sort ? enqueue_ray_sort(scene, s, in, counters, num_sms, stream) : s;
                 if ((e = launch_extend(scene, se, in, count, counters, extend_grid, stream, ev, true,
                                        c == 0 ? packet_forms : 0u)) != cudaSuccess)
                     return e;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                        shade<<<shade_blocks, 128, 0, stream>>>(scene, bg, ss, in, counters);
+                launch_chained(shade, shade_blocks, stream, scene, bg, ss, in, counters);
                 if (nee == kNeeDeferred)
                     enqueue_shadow_stage<2>(scene, DevCamera{}, FrameBuffers{}, RenderParams{}, bg, ss, b.rng, out, 0u,
                                             0u, counters, shadow_grid, shade_blocks, stream);

@@ -84,10 +84,8 @@ cudaError_t wavefront_alloc_nee(WavefrontState &s);
 constexpr uint32_t kChunkIterations = 8;
 struct ChunkGraph {
     cudaGraphExec_t exec = nullptr;
-    cudaEvent_t events[2 * kChunkIterations] = {};  // start/stop of each extend launch inside the graph
     std::vector<unsigned char> key;                 // kernel parameters the graph was captured with
     bool enabled = true;
-    bool timed = false;  // captured with the timing events
     uint32_t replays = 0, captures = 0;
 };
 void chunk_graph_free(ChunkGraph &g);
