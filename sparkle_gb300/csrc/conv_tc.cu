@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "chained_launch.cuh"
 #include "conv_tc.cuh"
 #include "tc_common.cuh"
 
@@ -188,6 +189,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         tma_prefetch_desc(&tmx);
         tma_prefetch_desc(&tmw);
     }
+    let_next_kernel_in();
+    after_previous_kernel();
     if (warp == 0) tmem_alloc(tmem_slot, ncols);
     tc_fence_before();
     __syncthreads();
@@ -373,6 +376,8 @@ __global__ void __launch_bounds__(kResThreads, kResCtas)
         mbar_init(wfull, 1);
         fence_mbar_init();
     }
+    let_next_kernel_in();
+    after_previous_kernel();
     if (warp == 0) tmem_alloc(tmem_slot, ncols);
     if (threadIdx.x < P.cout) bias[threadIdx.x] = P.out_spec.bias ? P.out_spec.bias[threadIdx.x] : 0.f;
     tc_fence_before();
@@ -976,8 +981,7 @@ cudaError_t forward_resident(const NhwcView &x, const void *w, uint32_t cout, co
     if (smem == 0) return cudaErrorInvalidConfiguration;
     const uint32_t grid = std::min(P.tiles, plan.ctas * static_cast<uint32_t>(device_sms()));
     auto *kern = P.out_spec.pool ? k_conv_res<true> : k_conv_res<false>;
-    kern<<<grid, kResThreads, smem, stream>>>(tmx, tmw, tmy, P);
-    return cudaGetLastError();
+    return launch_chained_if(epi.chained, kern, grid, kResThreads, smem, stream, tmx, tmw, tmy, P);
 }
 
 }  // namespace
@@ -1067,8 +1071,8 @@ cudaError_t conv3x3_forward(const NhwcView &x, const void *w, uint32_t cout, con
     const size_t smem = launch_smem(P.stages * P.stage_bytes + kFwdExtra, tmem_columns(mt * cout));
     if (smem == 0) return cudaErrorInvalidConfiguration;
     auto *kern = P.out_spec.pool ? k_conv_fwd<true> : k_conv_fwd<false>;
-    kern<<<static_cast<unsigned>(tiles), kFwdThreads, smem, stream>>>(tmx, tmw, tmy, P);
-    return cudaGetLastError();
+    return launch_chained_if(epi.chained, kern, static_cast<unsigned>(tiles), kFwdThreads, smem, stream, tmx, tmw, tmy,
+                             P);
 }
 
 #ifndef SPK_CONV_WGRAD_TMA

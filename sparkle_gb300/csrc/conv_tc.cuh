@@ -33,6 +33,7 @@ struct ConvEpilogue {
     NhwcView mask{};              // optional: multiply by (mask > 0) (ReLU backward of the layer below)
     // optional: also write the 2x2 average pooling of the (BF16) output, dense [n][h/2][w/2][cout] (h, w even)
     void *pool = nullptr;
+    bool chained = true;  // may start while the kernel before it in the stream ends (chained_launch.cuh)
 };
 
 // y = conv3x3(x, w) over geometry g. `w` is bf16 [cout][9][cin]. `err` is a device word for error bits.

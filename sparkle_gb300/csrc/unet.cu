@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "chained_launch.cuh"
 #include "conv_tc.cuh"
 #include "fault.h"
 #include "spk_denoise.h"
@@ -140,6 +141,7 @@ __device__ __forceinline__ float relu_mask(float ref) { return ref > 0.f ? 1.f :
 
 // features fp32 [n][h][w][10] -> X0 bf16 [n][hp][wp][32], edge replication into the padding. Rows: n * hp.
 __global__ void k_input(const float *feat, bf16 *x0, uint32_t n, uint32_t h, uint32_t w, uint32_t hp, uint32_t wp) {
+    let_next_kernel_in();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;  // (column, channel group)
     if (j >= wp * (kInPad / 8u)) return;
     const uint32_t grp = j % (kInPad / 8u), x = j / (kInPad / 8u);
@@ -160,6 +162,8 @@ __global__ void k_input(const float *feat, bf16 *x0, uint32_t n, uint32_t h, uin
 // Nearest 2x upsampling: src [n][h][w][c] (dense) -> dst view [n][2h][2w] (ld_d, first c channels). Rows: n * h; each
 // thread reads its 8 channels once and writes them to the four fine pixels.
 __global__ void k_upsample(const bf16 *src, bf16 *dst, uint32_t ld_d, uint32_t n, uint32_t h, uint32_t w, uint32_t c) {
+    let_next_kernel_in();
+    after_previous_kernel();
     const uint32_t cg = c / 8, j = blockIdx.x * blockDim.x + threadIdx.x;  // (column, channel group)
     if (j >= w * cg) return;
     const uint32_t g = j % cg, x = j / cg;
@@ -177,6 +181,8 @@ __global__ void k_upsample(const bf16 *src, bf16 *dst, uint32_t ld_d, uint32_t n
 // Upsampling backward + ReLU mask: dst[q][ch] = (sum of the 4 children of q in src view) * (ref[q] > 0). Rows: n * h.
 __global__ void k_upsample_bwd(const bf16 *src, uint32_t ld_s, const bf16 *ref, uint32_t ld_r, bf16 *dst, uint32_t n,
                                uint32_t h, uint32_t w, uint32_t c) {
+    let_next_kernel_in();
+    after_previous_kernel();
     const uint32_t cg = c / 8, j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= w * cg) return;
     const uint32_t g = j % cg, x = j / cg;
@@ -203,6 +209,8 @@ __global__ void k_upsample_bwd(const bf16 *src, uint32_t ld_s, const bf16 *ref, 
 // dst[p][ch] = (gpool[parent(p)][ch] / 4 + skip[p][ch]) * (ref[p][ch] > 0). Rows: n * h (h even).
 __global__ void k_pool_bwd(const bf16 *gpool, const bf16 *skip, uint32_t ld_skip, const bf16 *ref, uint32_t ld_r,
                            bf16 *dst, uint32_t n, uint32_t h, uint32_t w, uint32_t c) {
+    let_next_kernel_in();
+    after_previous_kernel();
     const uint32_t cg = c / 8, j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= w * cg) return;
     const uint32_t g = j % cg, x = j / cg;
@@ -221,6 +229,8 @@ __global__ void k_pool_bwd(const bf16 *gpool, const bf16 *skip, uint32_t ld_skip
 // d = expm1(o), L = mean((d - t)^2 / (t^2 + 0.01)), dL/do = 2 (d - t) / (t^2 + 0.01) * exp(o) / (3P).
 __global__ void k_loss(const bf16 *out, const float *target, bf16 *gout, uint32_t n, uint32_t h, uint32_t w,
                        double *loss_sum) {
+    let_next_kernel_in();
+    after_previous_kernel();
     const size_t p = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t total = static_cast<size_t>(n) * h * w;
     float l = 0.f;
@@ -330,6 +340,8 @@ __global__ void k_refresh_weights(const __grid_constant__ WeightTable T, const f
 
 // OUT [n][hp][wp][32] -> rgb float4 [n][h][w] (expm1 of the log1p prediction). Rows: n * h.
 __global__ void k_decode(const bf16 *out, float4 *dst, uint32_t n, uint32_t h, uint32_t w, uint32_t hp, uint32_t wp) {
+    let_next_kernel_in();
+    after_previous_kernel();
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= w) return;
     for (size_t row = blockIdx.y; row < static_cast<size_t>(n) * h; row += gridDim.y) {
@@ -607,12 +619,18 @@ cudaError_t conv_fwd(spk_denoiser *dn, uint32_t li, const NhwcView &x, const Nhw
     return conv3x3_forward(x, dn->wb.p + L.wb_off, L.cout, y, g, epi, dn->err.p, dn->stream);
 }
 
+// Whether the input gradients' kernels start while the one before them ends. Blocks that wait hold shared memory that
+// the weight gradients on the side stream could use: 1 x 64 x 64 pixels 577 -> 494 us, 16 x 128 x 128 1075 -> 1071,
+// 16 x 160 x 160 1407 -> 1419 with every level's chained. `g`: the level's own geometry.
+bool chain_backward(const ConvGeom &g) { return static_cast<size_t>(g.n) * g.h * g.w <= (1u << 18); }
+
 // Input gradient of layer li: dx = conv(dy, wt), optionally times (mask > 0).
 cudaError_t conv_dgrad(spk_denoiser *dn, uint32_t li, const NhwcView &dy, const NhwcView &dx, const ConvGeom &g,
                        const NhwcView *mask) {
     const Layer &L = dn->layers[li];
     ConvEpilogue epi;
     if (mask) epi.mask = *mask;
+    epi.chained = chain_backward(g);
     return conv3x3_forward(dy, dn->wt.p + L.wb_off, L.cin, dx, g, epi, dn->err.p, dn->stream);
 }
 
@@ -657,10 +675,11 @@ cudaError_t forward(spk_denoiser *dn, const float *feat, uint32_t n, uint32_t h,
     NhwcView up = dense(dn->eb4.p, kW[4]);
     for (int l = 3; l >= 0; --l) {
         const ConvGeom c = G(l + 1);
-        k_upsample<<<row_grid(static_cast<size_t>(c.w) * (up.channels / 8), static_cast<size_t>(n) * c.h), kGlueThreads, 0,
-                     dn->stream>>>(static_cast<const bf16 *>(up.ptr), dn->cat[l].p, cat_channels(l), n, c.h, c.w,
-                                   up.channels);
-        if ((e = conv_fwd(dn, dec_a(l), dense(dn->cat[l].p, cat_channels(l)), dense(dn->da[l].p, kW[l]), G(l))) !=
+        if ((e = launch_chained(k_upsample,
+                                row_grid(static_cast<size_t>(c.w) * (up.channels / 8), static_cast<size_t>(n) * c.h),
+                                kGlueThreads, 0, dn->stream, static_cast<const bf16 *>(up.ptr), dn->cat[l].p,
+                                cat_channels(l), n, c.h, c.w, up.channels)) != cudaSuccess ||
+            (e = conv_fwd(dn, dec_a(l), dense(dn->cat[l].p, cat_channels(l)), dense(dn->da[l].p, kW[l]), G(l))) !=
                 cudaSuccess ||
             (e = conv_fwd(dn, dec_b(l), dense(dn->da[l].p, kW[l]), dense(dn->db[l].p, kW[l]), G(l))) != cudaSuccess)
             return e;
@@ -701,8 +720,11 @@ cudaError_t backward_launches(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_
         const uint32_t cu = kW[l + 1];
         const bf16 *ref = l < 3 ? dn->db[l + 1].p : dn->eb4.p;
         bf16 *dst = l < 3 ? dn->g_db[l + 1].p : dn->g_eb[4].p;
-        k_upsample_bwd<<<row_grid(static_cast<size_t>(c.w) * (cu / 8), static_cast<size_t>(n) * c.h), kGlueThreads, 0,
-                         dn->stream>>>(dn->g_cat[l].p, cat_channels(l), ref, cu, dst, n, c.h, c.w, cu);
+        if ((e = launch_chained_if(chain_backward(c), k_upsample_bwd,
+                                row_grid(static_cast<size_t>(c.w) * (cu / 8), static_cast<size_t>(n) * c.h),
+                                kGlueThreads, 0, dn->stream, dn->g_cat[l].p, cat_channels(l), ref, cu, dst, n, c.h, c.w,
+                                cu)) != cudaSuccess)
+            return e;
     }
     // encoder, bottom up
     for (int l = 4; l >= 0; --l) {
@@ -720,9 +742,12 @@ cudaError_t backward_launches(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_
         const ConvGeom f = G(l - 1);
         const uint32_t cf = kW[l - 1];
         const NhwcView eo = enc_out(dn, l - 1);
-        k_pool_bwd<<<row_grid(static_cast<size_t>(f.w) * (cf / 8), static_cast<size_t>(n) * f.h), kGlueThreads, 0,
-                     dn->stream>>>(dn->g_pool[l - 1].p, dn->g_cat[l - 1].p + kW[l], cat_channels(l - 1),
-                                   static_cast<const bf16 *>(eo.ptr), eo.ld, dn->g_eb[l - 1].p, n, f.h, f.w, cf);
+        if ((e = launch_chained_if(chain_backward(f), k_pool_bwd,
+                                row_grid(static_cast<size_t>(f.w) * (cf / 8), static_cast<size_t>(n) * f.h),
+                                kGlueThreads, 0, dn->stream, dn->g_pool[l - 1].p, dn->g_cat[l - 1].p + kW[l],
+                                cat_channels(l - 1), static_cast<const bf16 *>(eo.ptr), eo.ld, dn->g_eb[l - 1].p, n,
+                                f.h, f.w, cf)) != cudaSuccess)
+            return e;
     }
     k_bias_grads<<<bias.first[bias.count], 256, 0, dn->stream>>>(bias);
     return cudaGetLastError();
@@ -758,7 +783,9 @@ spk_status loss_and_grads(spk_denoiser *dn, const float *feat, const float *targ
     DN_TRY(cudaEventRecord(dn->ev0, dn->stream), "event");
     DN_TRY(forward(dn, feat, n, h, w, h, w), "forward");
     const size_t p0 = static_cast<size_t>(n) * h * w;
-    k_loss<<<blocks_for(p0, 256), 256, 0, dn->stream>>>(dn->out.p, target, dn->gout.p, n, h, w, dn->loss.p);
+    DN_TRY(launch_chained(k_loss, blocks_for(p0, 256), 256, 0, dn->stream, dn->out.p, target, dn->gout.p, n, h, w,
+                          dn->loss.p),
+           "loss");
     DN_TRY(backward(dn, n, h, w), "backward");
     double l = 0.0;
     DN_TRY(cudaMemcpyAsync(&l, dn->loss.p, sizeof(double), cudaMemcpyDeviceToHost, dn->stream), "loss read");
@@ -1062,9 +1089,9 @@ spk_status spk_dn_infer(spk_denoiser *dn, const float *d_features, uint32_t n, u
     if (dn->weights_dirty) DN_TRY(refresh_weights(dn), "weight conversion");
     DN_TRY(cudaEventRecord(dn->ev0, dn->stream), "event");
     DN_TRY(forward(dn, d_features, n, h, w, hp, wp), "forward");
-    k_decode<<<row_grid(w, static_cast<size_t>(n) * h), kGlueThreads, 0, dn->stream>>>(
-        dn->out.p, reinterpret_cast<float4 *>(d_out), n, h, w, hp, wp);
-    DN_TRY(cudaGetLastError(), "decode");
+    DN_TRY(launch_chained(k_decode, row_grid(w, static_cast<size_t>(n) * h), kGlueThreads, 0, dn->stream, dn->out.p,
+                          reinterpret_cast<float4 *>(d_out), n, h, w, hp, wp),
+           "decode");
     DN_TRY(cudaEventRecord(dn->ev1, dn->stream), "event");
     return SPK_OK;
 }

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "wavefront.cuh"
+#include "chained_launch.cuh"
 #include "fault.h"
 
 #ifndef SPK_SHADE_MIN_BLOCKS
@@ -32,38 +33,16 @@ constexpr int kPacketQueue = 8;
 constexpr int kPacket2Queue = 9;
 constexpr int kNextItem = 10;  // next (frame, pixel) sample item to hand out
 
-// First statement of every kernel that launch_chained starts: from here on the kernel before is complete and its
-// writes are visible.
-__device__ __forceinline__ void after_previous_kernel() { cudaGridDependencySynchronize(); }
-
-// Lets the kernel after this one be launched: its blocks take the places of those that leave and wait in
-// after_previous_kernel. A walk's grid fills the SMs and spreads evenly however it comes in; the shading grids do
+// A walk's grid fills the SMs and spreads evenly however its blocks come in (chained_launch.cuh); the shading grids do
 // not, and shading many paths from uneven places costs more than the launch, so a walk of more than kEarlyRays rays
 // lets them in as its last blocks leave (1080p, 64 samples: 101.07 ms with all let in early, 100.63 so, 100.78 with
 // plain launches; 335 x 202, 1 sample: 494, 492 and 552 us with an event node on each side of the walks).
-__device__ __forceinline__ void let_next_kernel_in() { cudaTriggerProgrammaticLaunchCompletion(); }
 constexpr unsigned long long kEarlyRays = 1ull << 20;
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
-}
-
-// Starts a kernel of the extend / shade loop (128 threads a block) without waiting for the launch latency and the last
-// block of the kernel before it.
-template <class... Params, class... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, cudaStream_t stream, const Args &...args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(128);
-    cfg.stream = stream;
-    cudaLaunchAttribute chained{};
-    chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    chained.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &chained;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
 template <int kKind>
@@ -1017,7 +996,7 @@ uint32_t pass_packet_forms(uint32_t frames, const WfTuning &tuning) {
 
 cudaError_t launch_extend(const DevScene &scene, const WavefrontState &s, int in, bool count, Counters *counters,
                           unsigned grid, cudaStream_t stream, LaunchEvents *ev, bool batch, uint32_t packet_forms) {
-    auto launch = [&](auto *kernel) { return launch_chained(kernel, grid, stream, scene, s, in, counters); };
+    auto launch = [&](auto *kernel) { return launch_chained(kernel, grid, 128, 0, stream, scene, s, in, counters); };
     cudaError_t e = cudaSuccess;
     if (ev) ev->before(stream);
     if (batch) {
@@ -1065,9 +1044,9 @@ void enqueue_shadow_stage(const DevScene &scene, const DevCamera &cam, const Fra
                           const BatchParams &b, const WavefrontState &s, uint32_t rng, int out_queue,
                           uint32_t frame_base, uint32_t total_items, Counters *counters, unsigned walk_grid,
                           unsigned shade_grid, cudaStream_t stream) {
-    launch_chained(k_wf_shadow<kMode == 2>, walk_grid, stream, scene, s, counters);
+    launch_chained(k_wf_shadow<kMode == 2>, walk_grid, 128, 0, stream, scene, s, counters);
     auto *acc = rng == 0 ? k_nee_accumulate<0, kMode> : k_nee_accumulate<1, kMode>;
-    launch_chained(acc, shade_grid, stream, cam, fbuf, p, scene, b, s, out_queue, frame_base, total_items, counters);
+    launch_chained(acc, shade_grid, 128, 0, stream, cam, fbuf, p, scene, b, s, out_queue, frame_base, total_items, counters);
 }
 
 }  // namespace
@@ -1177,7 +1156,7 @@ cudaError_t launch_render_wavefront(const DevScene &scene, const DevCamera &cam,
             ss = enqueue_material_sort(scene, se, in, counters, num_sms, stream);
             nl += 3;
         }
-        launch_chained(shade, shade_blocks, stream, scene, fbuf, p, ss, in, b, counters);
+        launch_chained(shade, shade_blocks, 128, 0, stream, scene, fbuf, p, ss, in, b, counters);
         ++nl;
         if (nee == kNeeDeferred) {
             enqueue_shadow_stage<0>(scene, cam, fbuf, p, BatchParams{}, ss, p.rng, out, 0u, 0u, counters, shadow_grid,
@@ -1263,7 +1242,7 @@ cudaError_t launch_render_multiframe(const DevScene &scene, const DevCamera &cam
                     return ce;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                launch_chained(shade, shade_blocks, stream, scene, cam, fbuf, p, ss, in, f0, total_items,
+                launch_chained(shade, shade_blocks, 128, 0, stream, scene, cam, fbuf, p, ss, in, f0, total_items,
                                together ? static_cast<int>(c) : -1, counters);
                 if (nee == kNeeDeferred)
                     enqueue_shadow_stage<1>(scene, cam, fbuf, p, BatchParams{}, ss, p.rng, out, f0, total_items,
@@ -1426,7 +1405,7 @@ cudaError_t launch_render_batch(const DevScene &scene, const BatchParams &b, con
                     return e;
                 const WavefrontState ss =
                     tuning.material_sort ? enqueue_material_sort(scene, se, in, counters, num_sms, stream) : se;
-                launch_chained(shade, shade_blocks, stream, scene, bg, ss, in, counters);
+                launch_chained(shade, shade_blocks, 128, 0, stream, scene, bg, ss, in, counters);
                 if (nee == kNeeDeferred)
                     enqueue_shadow_stage<2>(scene, DevCamera{}, FrameBuffers{}, RenderParams{}, bg, ss, b.rng, out, 0u,
                                             0u, counters, shadow_grid, shade_blocks, stream);
