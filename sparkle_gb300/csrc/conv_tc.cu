@@ -16,7 +16,8 @@
 //                  ReLU or ReLU-backward mask, BF16 pack, 16-byte stores.
 // Layers whose weights fit beside the ring, on images of several tiles per SM, go to k_conv_res instead: the
 // same MMAs from persistent CTAs that keep the weights.
-// Wgrad (one CTA per (128 rows of (tap, ci), pixel range)): TMA loads of the shifted input and the output
+// Wgrad, up to 64 output channels: k_conv_wgrad_rows, one CTA per (32 input channels, pixel range). Wider layers
+// (one CTA per (128 rows of (tap, ci), pixel range)): TMA loads of the shifted input and the output
 // gradient as they lie in NHWC memory (MN-major operands, 64-byte swizzle), MMAs that read them MN-major,
 // and the FP32 partial sums added to dw with atomics. (SPK_CONV_WGRAD_TMA=0 keeps the earlier form: all
 // threads gather and transpose both operands into K-major swizzled tiles.)
@@ -783,6 +784,132 @@ __global__ void __launch_bounds__(128, 1)
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// wgrad of narrow layers: one input box per column tap serves its three row taps
+// ------------------------------------------------------------------------------------------------
+// k_conv_wgrad_tma loads every pixel of x once per tap and dy once per M tile, 15 spans of 4 KB per 64 pixels of a
+// 32 -> 32 layer, and those loads are its time. Here a CTA takes one 32-channel chunk of x with all nine taps. Per K
+// block and column tap it loads the box {32 ch, tw, th + 2} whose rows 0.., 1.., 2.. are the operands of the three row
+// taps, and dy once: 22 KB instead of 60. The M tile of a column tap is four spans of 32 channels, each one row of the
+// box after the other (leading byte offset tw * 64, so the spans overlap); the fourth, a row tap that does not exist,
+// reads up to one row past the box, still inside the stage, and its accumulator rows are not written out. Three
+// accumulators of cout columns: up to 64 output channels two CTAs fit an SM. 16 x 128 x 128 pixels, 32 -> 32: 34 -> 17
+// us, 96 -> 32: 75 -> 30; 16 x 64 x 64, 64 -> 64: 20 -> 16, 160 -> 64: 37 -> 23. A third of the error against 64 bits:
+// each accumulator sums fewer pixels.
+constexpr uint32_t kWgrMaxCout = 64;
+constexpr uint32_t kWgrStages = 4;
+
+struct WgradRowsParams {
+    uint32_t n, h, w, cin, cout;
+    uint32_t tw, th, tiles_x, tiles_y;  // K-block pixel tile (64 pixels) and tiles per image row / column
+    uint32_t chunks;                    // cin / 32
+    uint32_t kblocks, ktotal;           // K blocks per CTA, and in all images
+    uint32_t stages, a_bytes, stage_bytes;
+    float *dw;
+    uint32_t *err;
+};
+
+__global__ void __launch_bounds__(128, 1)
+    k_conv_wgrad_rows(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmdy,
+                      WgradRowsParams P) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = align1024(smem_raw);
+    const uint32_t nst = P.stages, stage_bytes = P.stage_bytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + nst * stage_bytes);
+    uint64_t *full = bars, *empty = bars + kWgrStages, *accum = bars + 2 * kWgrStages;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kWgrStages + 1);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t ncols = tmem_columns(3u * P.cout);
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < nst; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(accum, 1);
+        fence_mbar_init();
+        tma_prefetch_desc(&tmx);
+        tma_prefetch_desc(&tmdy);
+    }
+    if (warp == 0) tmem_alloc(tmem_slot, ncols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    const uint32_t chunk = blockIdx.x % P.chunks, split = blockIdx.x / P.chunks;
+    const uint32_t kb0 = split * P.kblocks;
+    const uint32_t nkb = kb0 < P.ktotal ? min(P.kblocks, P.ktotal - kb0) : 0u;
+    const uint32_t cspans = P.cout / 32u;
+
+    if (warp == 0 && lane == 0) {
+        const uint32_t tx_bytes = 3u * P.a_bytes + cspans * kWgtSpanBytes;
+        for (uint32_t i = 0; i < nkb; ++i) {
+            const uint32_t s = i % nst, u = i / nst;
+            if (u > 0 && !mbar_wait(&empty[s], (u - 1) & 1u, P.err)) break;
+            uint32_t t = kb0 + i;
+            const uint32_t tx = t % P.tiles_x;
+            t /= P.tiles_x;
+            const uint32_t ty = t % P.tiles_y;
+            const int img = static_cast<int>(t / P.tiles_y);
+            const int x0 = static_cast<int>(tx * P.tw), y0 = static_cast<int>(ty * P.th);
+            uint8_t *a = smem + s * stage_bytes;
+            uint8_t *b = a + 3u * P.a_bytes;
+            mbar_arrive_expect_tx(&full[s], tx_bytes);
+            for (uint32_t dx3 = 0; dx3 < 3; ++dx3)
+                tma_load_4d(a + dx3 * P.a_bytes, &tmx, &full[s], static_cast<int>(chunk * 32u),
+                            x0 + static_cast<int>(dx3) - 1, y0 - 1, img);
+            for (uint32_t sp = 0; sp < cspans; ++sp)
+                tma_load_4d(b + sp * kWgtSpanBytes, &tmdy, &full[s], static_cast<int>(sp * 32u), x0, y0, img);
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = idesc_bf16(kTileM, P.cout, true, true);
+        const bool issue = elect_one();
+        bool ok = true;
+        for (uint32_t i = 0; i < nkb; ++i) {
+            const uint32_t s = i % nst, u = i / nst;
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], u & 1u, P.err));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t stage = smem_u32(smem + s * stage_bytes);
+            const uint32_t a = smem_desc_mn_sw64(stage, P.tw * 64u);
+            const uint32_t b = smem_desc_mn_sw64(stage + 3u * P.a_bytes, kWgtSpanBytes);
+#pragma unroll
+            for (uint32_t dx3 = 0; dx3 < 3; ++dx3)
+#pragma unroll
+                for (uint32_t k16 = 0; k16 < kWgtPix / 16u; ++k16)
+                    mma_bf16(tmem + dx3 * P.cout, a + dx3 * (P.a_bytes / 16u) + k16 * 64u, kDescHiSw64, b + k16 * 64u,
+                             kDescHiSw64, idesc, i | k16, issue);
+            mma_commit(&empty[s], issue);
+        }
+        if (ok && nkb > 0) mma_commit(accum, issue);
+    }
+    __syncwarp();
+
+    bool ready = nkb > 0 && mbar_wait(accum, 0, P.err);
+    ready = __all_sync(0xFFFFFFFFu, ready);
+    tc_fence_after();
+    if (ready && warp < 3) {  // warp = row tap, lane = channel of the chunk
+        for (uint32_t j = 0; j < 3u * P.cout / 16u; ++j) {
+            uint32_t v[16];
+            tmem_ld16(tmem + ((warp * 32u) << 16) + j * 16u, v);
+            const uint32_t dx3 = j * 16u / P.cout, co = j * 16u - dx3 * P.cout;
+            float *dst = P.dw + (static_cast<size_t>(co) * 9u + warp * 3u + dx3) * P.cin + chunk * 32u + lane;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float f = __uint_as_float(v[e]);
+                if (f != 0.f) atomicAdd(dst + static_cast<size_t>(e) * 9u * P.cin, f);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, ncols);
+    }
+}
+
 __global__ void k_transpose_weights(const __nv_bfloat16 *w, __nv_bfloat16 *wt, uint32_t cout, uint32_t cin) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;  // index into wt [cin][9][cout]
     if (i >= cout * cin * 9u) return;
@@ -1135,6 +1262,64 @@ cudaError_t wgrad_tma(const NhwcView &x, const NhwcView &dy, float *dw, const Co
     k_conv_wgrad_tma<<<static_cast<unsigned>(splits * P.m_tiles), 128, smem, stream>>>(tmx, tmdy, P);
     return cudaGetLastError();
 }
+// Weight gradient of a layer of at most kWgrMaxCout output channels.
+cudaError_t wgrad_rows(const NhwcView &x, const NhwcView &dy, float *dw, const ConvGeom &g, uint32_t *err,
+                       cudaStream_t stream) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return cudaErrorNotSupported;
+    WgradRowsParams P{};
+    P.n = g.n;
+    P.h = g.h;
+    P.w = g.w;
+    P.cin = x.channels;
+    P.cout = dy.channels;
+    P.tw = g.w >= 16u ? 16u : 8u;
+    P.th = kWgtPix / P.tw;
+    P.tiles_x = (g.w + P.tw - 1) / P.tw;
+    P.tiles_y = (g.h + P.th - 1) / P.th;
+    P.chunks = P.cin / 32u;
+    const unsigned long long ktotal = static_cast<unsigned long long>(P.tiles_x) * P.tiles_y * g.n;
+    if (ktotal > 0x7FFFFFFFull) return cudaErrorInvalidValue;
+    P.ktotal = static_cast<uint32_t>(ktotal);
+    P.dw = dw;
+    P.err = err;
+    P.a_bytes = 64u * P.tw * (P.th + 2u);
+    // (a fourth span reads one row past the third box: into dy, which has at least 64 rows)
+    P.stage_bytes = (3u * P.a_bytes + (P.cout / 32u) * kWgtSpanBytes + 1023u) & ~1023u;
+    // The ring of two CTAs per SM.
+    constexpr uint32_t kExtra = 1024u + 256u;
+    P.stages = std::min<uint32_t>(kWgrStages, (228u * 1024u / 2u - 1024u - kExtra) / P.stage_bytes);
+    CUtensorMap tmx, tmdy;
+    const NhwcView *views[2] = {&x, &dy};
+    CUtensorMap *maps[2] = {&tmx, &tmdy};
+    for (int k = 0; k < 2; ++k) {
+        const NhwcView &v = *views[k];
+        const cuuint64_t dims[4] = {v.channels, g.w, g.h, g.n};
+        const cuuint64_t strides[3] = {static_cast<cuuint64_t>(v.ld) * 2u, static_cast<cuuint64_t>(v.ld) * 2u * g.w,
+                                       static_cast<cuuint64_t>(v.ld) * 2u * g.w * g.h};
+        const cuuint32_t box[4] = {32u, P.tw, k == 0 ? P.th + 2u : P.th, 1u};
+        const cuuint32_t es[4] = {1u, 1u, 1u, 1u};
+        if (enc(maps[k], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, v.ptr, dims, strides, box, es,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    // About two CTAs per SM in total, at least 2 K blocks each. (An M tile of k_conv_wgrad_tma takes 8 or more: there
+    // each split has 3 to 9 CTAs, here one.)
+    static const int sms = device_sms();
+    unsigned long long splits = std::max<unsigned long long>(1ull, (2ull * sms) / P.chunks);
+    splits = std::max<unsigned long long>(1ull, std::min<unsigned long long>(splits, (ktotal + 1) / 2));
+    P.kblocks = static_cast<uint32_t>((ktotal + splits - 1) / splits);
+    splits = (ktotal + P.kblocks - 1) / P.kblocks;
+    const size_t smem = launch_smem(P.stages * P.stage_bytes + kExtra, tmem_columns(3u * P.cout));
+    if (smem == 0 || P.stages < 2) return cudaErrorInvalidConfiguration;
+    static std::once_flag attr;
+    std::call_once(attr, [] {
+        cudaFuncSetAttribute(k_conv_wgrad_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+    });
+    k_conv_wgrad_rows<<<static_cast<unsigned>(splits * P.chunks), 128, smem, stream>>>(tmx, tmdy, P);
+    return cudaGetLastError();
+}
 }  // namespace
 
 cudaError_t conv3x3_wgrad(const NhwcView &x, const NhwcView &dy, float *dw, const ConvGeom &g, uint32_t *err,
@@ -1142,7 +1327,9 @@ cudaError_t conv3x3_wgrad(const NhwcView &x, const NhwcView &dy, float *dw, cons
     if (x.channels == 0 || x.channels % 32u || dy.channels == 0 || dy.channels % 32u || dy.channels > kMaxCout ||
         x.ld % 8u || dy.ld % 8u || !aligned16(x.ptr) || !aligned16(dy.ptr) || g.n == 0 || g.h == 0 || g.w == 0)
         return cudaErrorInvalidValue;
-    if (SPK_CONV_WGRAD_TMA) return wgrad_tma(x, dy, dw, g, err, stream);
+    if (SPK_CONV_WGRAD_TMA)
+        return dy.channels <= kWgrMaxCout ? wgrad_rows(x, dy, dw, g, err, stream)
+                                          : wgrad_tma(x, dy, dw, g, err, stream);
     WgradParams P{};
     P.n = g.n;
     P.h = g.h;

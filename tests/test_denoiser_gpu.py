@@ -216,3 +216,22 @@ def test_fallback_tiles(dn):
     mask = np.ones((h, w), bool)
     mask[16:32, 32:48] = False
     np.testing.assert_array_equal(got[mask], den[mask])
+
+
+@pytest.mark.parametrize("cin,cout", [(32, 32), (96, 32), (32, 64), (160, 64)])
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (1, 4, 16), (3, 5, 17), (1, 9, 8), (2, 7, 15), (2, 33, 47), (5, 64, 64)])
+def test_conv_wgrad_narrow(dn, n, h, w, cin, cout):
+    """Layers of at most 64 output channels share an input box between row taps: one to many K blocks, ragged
+    pixel tiles of 16 x 4 and 8 x 8, channel slices of wider buffers (whose other channels are NaN)."""
+    rng = np.random.default_rng(h * w + cin)
+    x = unet.to_bf16(rng.standard_normal((n, h, w, cin)).astype(np.float32))
+    gy = unet.to_bf16(rng.standard_normal((n, h, w, cout)).astype(np.float32))
+    xt = torch.full((n, h, w, cin + 32), float("nan"), dtype=torch.bfloat16, device="cuda")
+    gt = torch.full((n, h, w, cout + 32), float("nan"), dtype=torch.bfloat16, device="cuda")
+    xt[..., 8:8 + cin] = bf16_tensor(x)
+    gt[..., 16:16 + cout] = bf16_tensor(gy)
+    dw = torch.ones((cout, 3, 3, cin), dtype=torch.float32, device="cuda")
+    dn.conv3x3(2, xt[..., 8:], cin, None, gt[..., 16:], cout, n, h, w, x_ld=cin + 32, y_ld=cout + 32, dw=dw)
+    ref = 1.0 + unet.conv3x3_wgrad(x, gy).astype(np.float64)
+    got = dw.cpu().numpy().astype(np.float64)
+    assert np.linalg.norm(got - ref) <= 1e-3 * np.linalg.norm(ref)
