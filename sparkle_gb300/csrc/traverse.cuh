@@ -73,7 +73,7 @@ static_assert(kPacketSiblings >= 1 && kPacketSiblings <= 4, "one to four 8-lane 
 // 65536 + byte `c` of `word`: the byte, times 128, added to the bits of 65536.f (whose last place is 1/128). The byte dot
 // product does it in one instruction of the FMA pipe, where a byte permute, or an extraction and a conversion, would
 // go to the ALU pipe, the walk's busiest (it also takes the slab minima and maxima).
-__device__ __forceinline__ float plane(uint32_t word, int c) {
+__device__ __forceinline__ float raised_plane(uint32_t word, int c) {
     return __uint_as_float(__dp4a(word, 128u << (8 * c), 0x47800000u));
 }
 // Packed single-precision fused multiply-add (the halves rounded as fmaf rounds them).
@@ -87,6 +87,14 @@ __device__ __forceinline__ void fma_f2(unsigned long long a, unsigned long long 
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+}
+
+// Bytes `c` and `c` + 1 of `word` as floats: 65536 is taken off again two at a time, without rounding.
+__device__ __forceinline__ unsigned long long planes_f2(uint32_t word, int c) {
+    const unsigned long long raised = pack_f2(raised_plane(word, c), raised_plane(word, c + 1));
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(raised), "l"(pack_f2(-65536.f, -65536.f)));
+    return d;
 }
 
 struct TraceResult {
@@ -105,26 +113,16 @@ struct LevelRay {
     uint32_t oct;  // bit k set when direction component k is negative
 };
 
-// Reciprocal for the slab test; a component with |d| <= FLT_EPSILON gets +-2^92 so that
+// Reciprocal for the slab test, correctly rounded; a component with |d| <= FLT_EPSILON gets +-2^100 so that
 // (bound - o) * inv keeps its exact sign without overflowing (an exact containment test on that axis).
-// kExact: correctly rounded (the packet walk's interval bounds carry no slack for it); otherwise the hardware's
-// approximate reciprocal (relative error <= 2^-23, part of visit_slots's slack).
-template <bool kExact>
 __device__ __forceinline__ float slab_inverse(float x) {
-    float r;
-    if (kExact) {
-        r = 1.f / x;
-    } else {
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    }
-    return fabsf(x) <= 1.1920928955078125e-07f ? copysignf(0x1p92f, x) : r;
+    return fabsf(x) <= 1.1920928955078125e-07f ? copysignf(0x1p100f, x) : 1.f / x;
 }
 
-template <bool kExact = false>
 __device__ __forceinline__ void setup_level(LevelRay &r, f3 o, f3 d) {
     r.o = o;
     r.d = d;
-    r.inv = mk3(slab_inverse<kExact>(d.x), slab_inverse<kExact>(d.y), slab_inverse<kExact>(d.z));
+    r.inv = mk3(slab_inverse(d.x), slab_inverse(d.y), slab_inverse(d.z));
     r.oct = (signbit(d.x) ? 1u : 0u) | (signbit(d.y) ? 2u : 0u) | (signbit(d.z) ? 4u : 0u);
 }
 
@@ -169,33 +167,26 @@ struct NodeHits {
 
 // Slab test of the 8 children of node `idx` against one ray, in pairs of children (packed multiply-adds).
 //
-// Bound: instruction issue and the ALU pipe, which runs at half the issue rate. Per visit of random nodes (a loop of
-// visits, counted by ncu): 277 warp instructions of which 159 on the ALU pipe with the byte planes converted one by one,
-// scalar or packed near / far, and every hit child's item bits assembled here; 194 and 81 now: the planes come from byte
-// dot products (FMA pipe), the packed operands are two children's (which needs no register moves), and only the slot
-// mask is built here (leaf items are decoded by the few rays that reach a leaf).
+// Bound: instruction issue and the ALU pipe, which runs at half the issue rate. With the byte planes converted one by
+// one and every hit child's item bits assembled here a visit took 277 warp instructions, 159 of them on the ALU pipe. The
+// planes come from byte dot products and packed adds (FMA pipe), the packed operands are two children's (which needs no
+// register moves), and only the slot mask is built here (leaf items are decoded by the few rays that reach a leaf).
 //
-// A child passes whenever its quantised box is entered within [0, tmax] in exact arithmetic. Per axis, with
-// inv = (1 / d)(1 + e), |e| <= 2^-23, the plane at byte q is at t = q a + o, a = scale * inv, o = (p - r.o) * inv,
-// evaluated as fma(65536 + q, a, o -+ slack - 65536 a). Errors: |o| (2^-22 from o itself, 3 * 2^-24 from the three later
-// roundings) and |a| (2 * 2^-8 from the roundings of o - 65536 a and its slack, below 2^-14 the rest), within the slack
-// of 2^-20 |o| + 2^-6 |a|. The slack also covers the rounding of the plain fma(q, a, o), so every box that form lets
-// pass passes here. (|o| is cut at 2^100 in the slack so that an overflowing o still misses: inf - inf would pass.)
+// The test is fma(q, a, o) on the plane bytes q, with a = scale * inv and o = (p - r.o) * inv, bit for bit the one of
+// walk_wide and of a packet's single rays. That matters: Moeller-Trumbore accepts rays that pass an edge by a rounding
+// error outside, so a triangle can be hit through a box that the exact ray misses, and a walk whose boxes are wider by a
+// slack, which would save the adds and the division (6% of a walk), finds hits that the others do not.
 __device__ __forceinline__ NodeHits visit_slots(const uint4 *__restrict__ nodes, uint32_t idx, const LevelRay &r,
                                                 float tmax) {
     const uint4 *np = nodes + static_cast<size_t>(idx) * 5;
     const uint4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
-    float a[3], near_o[3], far_o[3];
+    float a[3], o[3];
     const float p[3] = {__uint_as_float(n0.x), __uint_as_float(n0.y), __uint_as_float(n0.z)};
     const float ro[3] = {r.o.x, r.o.y, r.o.z}, ri[3] = {r.inv.x, r.inv.y, r.inv.z};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         a[k] = __uint_as_float(((n0.w >> (8 * k)) & 0xFFu) << 23) * ri[k];
-        const float o = (p[k] - ro[k]) * ri[k];
-        const float base = fmaf(-65536.f, a[k], o);
-        const float slack = fmaf(fminf(fabsf(o), 0x1p100f), 0x1p-20f, fabsf(a[k]) * 0x1p-6f);
-        near_o[k] = base - slack;
-        far_o[k] = base + slack;
+        o[k] = (p[k] - ro[k]) * ri[k];
     }
     NodeHits h{n1.x, n1.y, n0.w >> 24, 0u, {n1.z, n1.w}};
     const uint32_t lo[3][2] = {{n2.x, n2.y}, {n2.z, n2.w}, {n3.x, n3.y}};
@@ -214,9 +205,9 @@ __device__ __forceinline__ NodeHits visit_slots(const uint4 *__restrict__ nodes,
             float tn[3][2], tf[3][2];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const unsigned long long a2 = pack_f2(a[k], a[k]);
-                fma_f2(pack_f2(plane(nw[k], c), plane(nw[k], c + 1)), a2, pack_f2(near_o[k], near_o[k]), tn[k][0], tn[k][1]);
-                fma_f2(pack_f2(plane(fw[k], c), plane(fw[k], c + 1)), a2, pack_f2(far_o[k], far_o[k]), tf[k][0], tf[k][1]);
+                const unsigned long long a2 = pack_f2(a[k], a[k]), o2 = pack_f2(o[k], o[k]);
+                fma_f2(planes_f2(nw[k], c), a2, o2, tn[k][0], tn[k][1]);
+                fma_f2(planes_f2(fw[k], c), a2, o2, tf[k][0], tf[k][1]);
             }
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -760,7 +751,7 @@ __device__ __noinline__ uint32_t walk_wide(const DevScene &S, unsigned long long
         const uint32_t root = fetch(q, wo, wd, limit);
         if (kMode != kTraceOcclusion) limit = kFltMax;
         LevelRay ray;
-        setup_level<true>(ray, wo, wd);
+        setup_level(ray, wo, wd);
         TraceResult best{kFltMax, 0.f, 0.f, kInvalid, kInvalid};
         uint2 ng = make_uint2(root, root == kInvalid ? 0u : (1u << 24));  // inner children in visiting order, or TLAS items
         uint32_t left = S.walk_budget ? S.walk_budget : kMaxIterations;
@@ -899,7 +890,7 @@ __device__ __noinline__ uint32_t walk_wide(const DevScene &S, unsigned long long
                     if (ng.y != 0u) push(ng);
                     blas_sp = sp;
                     cur_inst = inst;
-                    setup_level<true>(ray, xform_point(I.minv, wo), xform_dir(I.minv, wd));
+                    setup_level(ray, xform_point(I.minv, wo), xform_dir(I.minv, wd));
                     ng = make_uint2(I.blas_root, 1u << 24);
                 }
             }
@@ -908,7 +899,7 @@ __device__ __noinline__ uint32_t walk_wide(const DevScene &S, unsigned long long
                 if (sp == blas_sp) blas_sp = -2;
                 ng = stack[--sp];
                 if (blas_sp == -2 && ng.y > 0x00FFFFFFu) {
-                    setup_level<true>(ray, wo, wd);
+                    setup_level(ray, wo, wd);
                     blas_sp = -1;
                 }
             }
@@ -1125,7 +1116,7 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                 wo[r] = o0;
                 wd[r] = d0;
             }
-            setup_level<true>(ray[r], wo[r], wd[r]);
+            setup_level(ray[r], wo[r], wd[r]);
             best[r] = TraceResult{kFltMax, 0.f, 0.f, kInvalid, kInvalid};
             tmax_box[r] = kFltMax;
 #if SPK_PACKET_WORLD_SMEM
@@ -1287,7 +1278,7 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
                         cur_inst = inst;
 #pragma unroll
                         for (int r = 0; r < kRays; ++r)
-                            setup_level<true>(ray[r], xform_point(I.minv, ray[r].o), xform_dir(I.minv, ray[r].d));
+                            setup_level(ray[r], xform_point(I.minv, ray[r].o), xform_dir(I.minv, ray[r].d));
                         const uint32_t entering = __ballot_sync(kAll, mine);  // not empty: the group had bit k
                         order = __shfl_sync(kAll, ray[0].oct, __ffs(entering) - 1);
                         packed = make_frustum(ray, order, frustum);
@@ -1304,9 +1295,9 @@ __device__ __forceinline__ void walk_packets(const DevScene &S, unsigned long lo
 #pragma unroll
                     for (int r = 0; r < kRays; ++r) {
 #if SPK_PACKET_WORLD_SMEM
-                        setup_level<true>(ray[r], world_o(r), world_d(r));
+                        setup_level(ray[r], world_o(r), world_d(r));
 #else
-                        setup_level<true>(ray[r], wo[r], wd[r]);
+                        setup_level(ray[r], wo[r], wd[r]);
 #endif
                     }
                     order = top_order;

@@ -55,3 +55,32 @@ def test_stacked_triangles_match_the_oracle(layers, count):
     sphere = ref["face"][ref["prim"] != INVALID] == INVALID  # (an any-hit query takes a sphere behind the ray too)
     assert not ((any_hit["prim"] == INVALID) & (ref["prim"] != INVALID)).any(), sphere.sum()
     ctx.close()
+
+
+def test_edge_rays_are_the_same_whatever_walks_them():
+    """Rays that leave an axis-aligned box from a point of its walls, nearly along them: whether Moeller-Trumbore
+    accepts a wall's edge, and whether the ray enters its flat box, are both decided by the last bit. A large launch
+    (a ray per lane) and small ones (a ray per warp) have to decide alike."""
+    scene, _ = scenes.cornell_box(0)
+    ctx = native.Context(0)
+    ctx.set_scene(scene)
+    lo, hi = (np.asarray(v, np.float32) for v in scene.world_bounds())
+    rng = np.random.default_rng(3)
+    n = 200_000
+    o = (lo + (hi - lo) * rng.random((n, 3))).astype(np.float32)
+    d = rng.standard_normal((n, 3))
+    axis, side = rng.integers(0, 3, n), rng.integers(0, 2, n)
+    rows = np.arange(n)
+    o[rows, axis] = np.where(side == 1, hi[axis], lo[axis])
+    d[rows, axis] = np.where(side == 1, 1, -1) * 10 ** rng.uniform(-7, -2, n)
+    near = (axis + 1) % 3  # close to a neighbouring wall, towards it
+    o[rows, near] = (lo[near] + (hi[near] - lo[near]) * 10 ** rng.uniform(-6, -2, n)).astype(np.float32)
+    d[rows, near] = -np.abs(d[rows, near])
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.concatenate([o, d.astype(np.float32)], 1).astype(np.float32)
+    whole = ctx.trace(rays)
+    for a in range(0, n, 8192):
+        part = ctx.trace(rays[a:a + 8192])
+        for f in ("t", "u", "v", "prim", "face"):
+            assert np.array_equal(whole[f][a:a + 8192].view(np.uint32), part[f].view(np.uint32)), (f, a)
+    ctx.close()
