@@ -347,7 +347,8 @@ spk_status spk_get_config(const spk_ctx *ctx, spk_config *out);
 /* Replaces `num_frames` calls of CPURenderer::Render (CPURenderer.cpp:119-208) on a static scene: per frame
  * the clear (if dirty), BasePass (:419-450), DenoisePass (:506-552) and ToneMappingPass (:565-576), with
  * the camera's cumulated-sample bookkeeping between frames (CameraRenderProxy.cpp:66-75). Asynchronous
- * with respect to the host: results are visible to spk_read_framebuffer / spk_synchronize. */
+ * with respect to the host: results are visible to spk_read_framebuffer / spk_synchronize. A call that fails
+ * leaves the accumulation as it was; one of more than 64 frames may have folded some and restarts it. */
 spk_status spk_render(spk_ctx *ctx, uint32_t num_frames);
 
 /* Copies the accumulated HDR frame buffer (`frame_buffer_`, H rows of W float4, row j = image row j from

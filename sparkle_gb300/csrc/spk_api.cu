@@ -1398,23 +1398,20 @@ static spk_status render_impl(spk_ctx *ctx, uint32_t num_frames) {
     if (wavefront && ctx->tuning.multi_frame && num_frames > 0) {
         // All frames in one regenerating wavefront: the per-frame bookkeeping runs ahead on the host, the kernels derive
         // each frame's weight and seed base from its start (the spatial fill, when on, runs per frame in the
-        // resolve over that frame's samples and first-hit normals).
-        FrameSchedule sched{0u, ctx->spp_eff, 0u, ctx->cfg.max_spp, ctx->dirty};
+        // resolve over that frame's samples and first-hit normals). It becomes the context's once everything is
+        // queued: a call that fails before that, by a status or an exception, has folded no frame, and leaves the
+        // accumulation, and a clear that is due, as they were.
+        uint32_t cumulated = ctx->dirty ? 0u : ctx->cumulated, pending = ctx->dirty ? 0u : ctx->pending;
+        uint32_t dispatched = ctx->dirty ? ctx->cfg.sample_offset : ctx->dispatched;
+        FrameSchedule sched{dispatched, ctx->spp_eff, 0u, ctx->cfg.max_spp, ctx->dirty};
         for (uint32_t f = 0; f < num_frames; ++f) {
-            if (ctx->dirty) {
-                ctx->cumulated = 0;
-                ctx->pending = 0;
-                ctx->dispatched = ctx->cfg.sample_offset;
-                ctx->dirty = false;
-            }
-            ctx->cumulated = std::min(ctx->cfg.max_spp, ctx->cumulated + ctx->pending);
-            if (f == 0) {
-                sched.seed_base = ctx->dispatched;
-                sched.cumulated = ctx->cumulated;
-            }
-            ctx->dispatched += ctx->spp_eff;
-            ctx->pending = ctx->spp_eff;
+            cumulated = std::min(ctx->cfg.max_spp, cumulated + pending);
+            if (f == 0) sched.cumulated = cumulated;
+            dispatched += ctx->spp_eff;
+            pending = ctx->spp_eff;
         }
+        // Several passes: an earlier one may have folded its frames when a later one fails, so a failure clears.
+        if (num_frames > kFramesPerPass) ctx->dirty = true;
         RenderParams p{0u, ctx->cfg.bounce, ctx->cfg.rng, ctx->cfg.seed, ctx->cfg.spatial_denoise, ctx->cfg.enable_nee};
         uint32_t launches = 0;
         ctx->chunk_graph.enabled = ctx->tuning.cuda_graph != 0;
@@ -1424,18 +1421,19 @@ static spk_status render_impl(spk_ctx *ctx, uint32_t num_frames) {
         const uint64_t npix = static_cast<uint64_t>(ctx->cfg.width) * ctx->cfg.height;
         const uint64_t per_pixel = std::min<uint64_t>({ctx->tuning.path_slots_per_pixel, num_frames, kFramesPerPass});
         const uint64_t slots = std::max<uint64_t>(npix, std::min<uint64_t>(npix * per_pixel, kMaxPathSlots));
-        if (ctx->wf.capacity < slots && (e = wavefront_alloc(ctx->wf, static_cast<uint32_t>(slots))) != cudaSuccess) {
-            ctx->dirty = ctx->dirty || sched.clear;  // the resolve that would have cleared the buffer does not run
+        if (ctx->wf.capacity < slots && (e = wavefront_alloc(ctx->wf, static_cast<uint32_t>(slots))) != cudaSuccess)
             return cuda_fail(ctx, e, "path state allocation");
-        }
         e = launch_render_multiframe(ctx->scene, ctx->cam, fbuf, p, num_frames, sched, count, ctx->counters, ctx->wf,
                                      ctx->num_sms, ctx->stream, &launches, &ctx->launch_events, wf_tuning(ctx),
                                      &ctx->chunk_graph);
         if (e != cudaSuccess) {
-            ctx->dirty = ctx->dirty || sched.clear;
             const std::string what = std::string("multi-frame wavefront (") + wavefront_error_site() + ")";
             return cuda_fail(ctx, e, what.c_str());
         }
+        ctx->cumulated = cumulated;
+        ctx->pending = pending;
+        ctx->dispatched = dispatched;
+        ctx->dirty = false;
         ctx->launches_in_call = launches;
         if ((e = cudaEventRecord(ctx->ev_stop, ctx->stream)) != cudaSuccess) return cuda_fail(ctx, e, "event");
         ctx->last = spk_stats{};

@@ -90,6 +90,51 @@ def test_allocation_failures_are_reported_and_recovered(cornell, small_terrain):
     ctx.close()
 
 
+@pytest.mark.parametrize("frames,moved", [(3, False), (3, True), (65, False)])
+def test_a_failed_render_leaves_the_accumulation_as_it_was(cornell, frames, moved):
+    """Every device allocation of a render fails in turn (path state, light-sampling records, samples, normals). The
+    call repeated then gives the image and the sample counts of a context in which nothing failed: the frames before it
+    still count, or the clear that a moved camera asked for is still due. More than one pass (64 frames) starts over."""
+    cfg = dict(spp=4, bounce=4, seed=2, max_spp=1024, enable_nee=True, spatial_denoise=1)
+    other = scenes.make_camera(dict(cornell[1], position=(0.4, -1.2, 0.6)), 32, 24)
+
+    def context():
+        ctx = native.Context(0)
+        setup(ctx, cornell, 32, 24, **cfg)
+        return ctx
+
+    ref = context()
+    if frames <= 64:
+        ref.render(1)
+    if moved:
+        ref.set_camera(other)
+    ref.render(frames)
+    want, counts = ref.framebuffer(), ref.sample_counts()
+    ref.close()
+    failed = 0
+    for nth in range(1, 100):
+        ctx = context()
+        ctx.render(1)
+        if moved:
+            ctx.set_camera(other)
+        native.debug_fail_allocation(nth)
+        try:
+            ctx.render(frames)
+        except native.SpkError as e:
+            assert e.status == OOM
+            failed += 1
+            ctx.render(frames)
+        else:
+            native.debug_fail_allocation(0)
+            ctx.close()
+            break
+        assert ctx.sample_counts() == counts, nth
+        for got, exp in zip(ctx.framebuffer(), want):
+            assert np.array_equal(got.view(np.uint8), exp.view(np.uint8)), nth
+        ctx.close()
+    assert failed >= 4
+
+
 def test_walk_budget_sets_the_error_flag(small_terrain):
     ctx = native.Context(0)
     scene, _ = small_terrain
