@@ -84,3 +84,26 @@ def test_edge_rays_are_the_same_whatever_walks_them():
         for f in ("t", "u", "v", "prim", "face"):
             assert np.array_equal(whole[f][a:a + 8192].view(np.uint32), part[f].view(np.uint32)), (f, a)
     ctx.close()
+
+
+@pytest.mark.parametrize("layers", [1, 24, 200])
+@pytest.mark.parametrize("count", [1, 33, 12768, 12769, 34049])
+def test_any_hit_over_stacked_triangles_is_the_oracles(layers, count):
+    """Any-hit flags both ways: a hit missed, and a hit reported for a ray that has none (a queued triangle credited to
+    another lane's ray would do that). Half of the rays pass beside the stack."""
+    scene = stacked_triangles(layers)
+    rng = np.random.default_rng(1000 + count)
+    target = np.stack([rng.uniform(-5, 5, count), rng.uniform(-4, 5, count), rng.uniform(-3, 1, count)], 1)
+    origin = np.stack([rng.uniform(-3, 3, count), rng.uniform(-3, 3, count), np.where(rng.random(count) < 0.5, 6.0, -8.0)], 1)
+    d = target - origin
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = abi.rays_to_array(origin, d)
+    want, _ = oracle.OracleScene(scene).trace(rays, any_hit=True)
+    hit = want["prim"] != INVALID
+    assert count < 1000 or 0.2 < hit.mean() < 0.8
+    ctx = native.Context(0)
+    ctx.set_scene(scene)
+    got = ctx.trace(rays, any_hit=True)
+    assert ctx.stats()["error_flags"] == 0
+    assert np.array_equal(got["prim"] != INVALID, hit)
+    ctx.close()
