@@ -486,6 +486,7 @@ struct DnRange {
 
 struct spk_denoiser {
     int device = 0;
+    int sms = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;  // weight gradients, beside the chain of input gradients; idle between calls
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -619,18 +620,24 @@ cudaError_t conv_fwd(spk_denoiser *dn, uint32_t li, const NhwcView &x, const Nhw
     return conv3x3_forward(x, dn->wb.p + L.wb_off, L.cout, y, g, epi, dn->err.p, dn->stream);
 }
 
-// Whether the input gradients' kernels start while the one before them ends. Blocks that wait hold shared memory that
-// the weight gradients on the side stream could use: 1 x 64 x 64 pixels 577 -> 494 us, 16 x 128 x 128 1075 -> 1071,
-// 16 x 160 x 160 1407 -> 1419 with every level's chained. `g`: the level's own geometry.
-bool chain_backward(const ConvGeom &g) { return static_cast<size_t>(g.n) * g.h * g.w <= (1u << 18); }
+// Whether backward's input gradients and the kernels between them start while the one before them ends. A block that
+// waits holds the shared memory of an SM (a small grid's ring takes all of it), which the weight gradients on the side
+// stream then lack for as long: that costs more than the launches it hides once the finest level has tiles for more
+// than 3 in 10 of the SMs. Chained / not, us: 1 x 32 x 32 pixels 362 / 409, 1 x 64 x 64 (32 tiles) 382 / 415, 1 x 64 x 80
+// (40) 401 / 414, 1 x 80 x 80 (50) 424 / 415, 1 x 160 x 160 488 / 445, 16 x 128 x 128 858 / 798, 16 x 160 x 160 1111 / 1063.
+// Coarse levels alone chained is no better either (16 x 128 x 128 with those of at most 4096 pixels 809, of 16384 847).
+bool chain_backward(const spk_denoiser *dn, const ConvGeom &finest) {
+    constexpr size_t kTilePixels = 128;
+    return static_cast<size_t>(finest.n) * finest.h * finest.w * 10 <= 3 * kTilePixels * static_cast<size_t>(dn->sms);
+}
 
 // Input gradient of layer li: dx = conv(dy, wt), optionally times (mask > 0).
 cudaError_t conv_dgrad(spk_denoiser *dn, uint32_t li, const NhwcView &dy, const NhwcView &dx, const ConvGeom &g,
-                       const NhwcView *mask) {
+                       const NhwcView *mask, bool chained) {
     const Layer &L = dn->layers[li];
     ConvEpilogue epi;
     if (mask) epi.mask = *mask;
-    epi.chained = chain_backward(g);
+    epi.chained = chained;
     return conv3x3_forward(dy, dn->wt.p + L.wb_off, L.cin, dx, g, epi, dn->err.p, dn->stream);
 }
 
@@ -698,12 +705,13 @@ cudaError_t forward(spk_denoiser *dn, const float *feat, uint32_t n, uint32_t h,
 cudaError_t backward_launches(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_t wp) {
     cudaError_t e;
     auto G = [&](uint32_t l) { return ConvGeom{n, hp >> l, wp >> l}; };
+    const bool chained = chain_backward(dn, G(0));
     BiasTable bias{};
     // output layer
     const NhwcView db0 = dense(dn->db[0].p, kW[0]);
     if ((e = layer_grads(dn, bias, kOutLayer, db0, dense(dn->gout.p, kOutPad), G(0))) != cudaSuccess) return e;
-    if ((e = conv_dgrad(dn, kOutLayer, dense(dn->gout.p, kOutPad), dense(dn->g_db[0].p, kW[0]), G(0), &db0)) !=
-        cudaSuccess)
+    if ((e = conv_dgrad(dn, kOutLayer, dense(dn->gout.p, kOutPad), dense(dn->g_db[0].p, kW[0]), G(0), &db0,
+                        chained)) != cudaSuccess)
         return e;
     // decoder, level 0 upwards
     for (uint32_t l = 0; l < 4; ++l) {
@@ -711,16 +719,16 @@ cudaError_t backward_launches(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_
         const NhwcView gdb = dense(dn->g_db[l].p, kW[l]), gda = dense(dn->g_da[l].p, kW[l]);
         const NhwcView cat = dense(dn->cat[l].p, cat_channels(l)), gcat = dense(dn->g_cat[l].p, cat_channels(l));
         if ((e = layer_grads(dn, bias, dec_b(l), da, gdb, G(l))) != cudaSuccess ||
-            (e = conv_dgrad(dn, dec_b(l), gdb, gda, G(l), &da)) != cudaSuccess ||
+            (e = conv_dgrad(dn, dec_b(l), gdb, gda, G(l), &da, chained)) != cudaSuccess ||
             (e = layer_grads(dn, bias, dec_a(l), cat, gda, G(l))) != cudaSuccess ||
-            (e = conv_dgrad(dn, dec_a(l), gda, gcat, G(l), nullptr)) != cudaSuccess)
+            (e = conv_dgrad(dn, dec_a(l), gda, gcat, G(l), nullptr, chained)) != cudaSuccess)
             return e;
         // gradient of the upsampled input -> the level below's decoder output (or the bottleneck)
         const ConvGeom c = G(l + 1);
         const uint32_t cu = kW[l + 1];
         const bf16 *ref = l < 3 ? dn->db[l + 1].p : dn->eb4.p;
         bf16 *dst = l < 3 ? dn->g_db[l + 1].p : dn->g_eb[4].p;
-        if ((e = launch_chained_if(chain_backward(c), k_upsample_bwd,
+        if ((e = launch_chained_if(chained, k_upsample_bwd,
                                 row_grid(static_cast<size_t>(c.w) * (cu / 8), static_cast<size_t>(n) * c.h),
                                 kGlueThreads, 0, dn->stream, dn->g_cat[l].p, cat_channels(l), ref, cu, dst, n, c.h, c.w,
                                 cu)) != cudaSuccess)
@@ -731,18 +739,18 @@ cudaError_t backward_launches(spk_denoiser *dn, uint32_t n, uint32_t hp, uint32_
         const NhwcView ea = dense(dn->ea[l].p, kW[l]);
         const NhwcView geb = dense(dn->g_eb[l].p, kW[l]), gea = dense(dn->g_ea[l].p, kW[l]);
         if ((e = layer_grads(dn, bias, enc_b(l), ea, geb, G(l))) != cudaSuccess ||
-            (e = conv_dgrad(dn, enc_b(l), geb, gea, G(l), &ea)) != cudaSuccess)
+            (e = conv_dgrad(dn, enc_b(l), geb, gea, G(l), &ea, chained)) != cudaSuccess)
             return e;
         const NhwcView in = l == 0 ? dense(dn->x0.p, kInPad) : dense(dn->pool[l - 1].p, kW[l - 1]);
         if ((e = layer_grads(dn, bias, enc_a(l), in, gea, G(l))) != cudaSuccess) return e;
         if (l == 0) break;
         const NhwcView gpool = dense(dn->g_pool[l - 1].p, kW[l - 1]);
-        if ((e = conv_dgrad(dn, enc_a(l), gea, gpool, G(l), nullptr)) != cudaSuccess) return e;
+        if ((e = conv_dgrad(dn, enc_a(l), gea, gpool, G(l), nullptr, chained)) != cudaSuccess) return e;
         // gradient at the level above's encoder output: pooling backward + skip gradient, ReLU mask
         const ConvGeom f = G(l - 1);
         const uint32_t cf = kW[l - 1];
         const NhwcView eo = enc_out(dn, l - 1);
-        if ((e = launch_chained_if(chain_backward(f), k_pool_bwd,
+        if ((e = launch_chained_if(chained, k_pool_bwd,
                                 row_grid(static_cast<size_t>(f.w) * (cf / 8), static_cast<size_t>(n) * f.h),
                                 kGlueThreads, 0, dn->stream, dn->g_pool[l - 1].p, dn->g_cat[l - 1].p + kW[l],
                                 cat_channels(l - 1), static_cast<const bf16 *>(eo.ptr), eo.ld, dn->g_eb[l - 1].p, n,
@@ -813,6 +821,7 @@ spk_status spk_dn_create(int32_t device, uint64_t seed, spk_denoiser **out) {
     dn->nweights = weight_count(dn->layers);
     cudaError_t e;
     if ((e = cudaSetDevice(device)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&dn->sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&dn->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&dn->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&dn->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
