@@ -656,9 +656,10 @@ cudaError_t layer_grads(spk_denoiser *dn, BiasTable &bias, uint32_t li, const Nh
     bias.g[k] = static_cast<const bf16 *>(dy.ptr);
     bias.db[k] = dn->grads.p + L.b_off;
     bias.pixels[k] = static_cast<size_t>(g.n) * g.h * g.w;
-    // 16 pixels a thread (a block more than that only adds to the atomics), at most 304 blocks: two per SM
+    // 16 pixels a thread (a block more than that only adds to the atomics), at most two blocks per SM
     const size_t rows = 256u / (dy.channels / 8u);
-    const size_t blocks = std::min<size_t>((bias.pixels[k] + 16 * rows - 1) / (16 * rows), 304);
+    const size_t blocks =
+        std::min((bias.pixels[k] + 16 * rows - 1) / (16 * rows), 2 * static_cast<size_t>(dn->sms));
     bias.first[k + 1] = bias.first[k] + static_cast<uint32_t>(blocks);
     return cudaSuccess;
 }
