@@ -93,6 +93,7 @@ struct DevScene {
     uint32_t num_scenes;
     float box_lo[3];     // world bounds of all scenes (ray sort cells)
     float box_scale[3];  // 8 / extent per axis (0 for a flat axis)
+    uint32_t num_nodes;    // of all scenes, TLAS and BLASes
     uint32_t walk_budget;  // node steps a walk may take before it reports kErrIterationBudget; 0 = 2^20
 };
 

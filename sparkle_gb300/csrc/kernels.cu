@@ -12,13 +12,14 @@ namespace {
 // ------------------------------------------------------------------------------------------------
 // Ray-set query: persistent warps pull rays from a global counter and refill idle lanes.
 // ------------------------------------------------------------------------------------------------
-template <int kMode, bool kCount>
-__global__ void __launch_bounds__(128, SPK_WALK_MIN_BLOCKS) k_trace(const __grid_constant__ DevScene S, const float *__restrict__ rays, uint64_t n,
-                                                  spk_hit_dev *__restrict__ hits, Counters *counters) {
+template <int kMode, bool kCount, bool kDirect>
+__global__ void __launch_bounds__(128, SPK_WALK_MIN_BLOCKS)
+    k_trace(const __grid_constant__ DevScene S, const float *__restrict__ rays, uint64_t n,
+            spk_hit_dev *__restrict__ hits, Counters *counters) {
     uint32_t err = 0;
     TraceCounts tc;
     const uint32_t root = S.tlas_root;
-    walk_rays<kMode, kCount>(
+    walk_rays<kMode, kCount, kDirect>(
         S, &counters->queue_counters[0], n, kFltMax, err, &tc,
         [rays, root](unsigned long long q, f3 &o, f3 &d, float &) {
             const float *r = rays + q * 6;
@@ -164,17 +165,26 @@ cudaError_t launch_trace(const DevScene &scene, const float *rays, uint64_t n, v
     auto *h = static_cast<spk_hit_dev *>(hits);
     const unsigned g = static_cast<unsigned>(blocks);
     if (ev) ev->before(stream);
+    // In a scene of few nodes most lanes reach a leaf in the same step: queueing its triangles gains no lanes, while each
+    // of them is taken into its instance's space again, and a walk that a hit would end goes on until the queue is
+    // tested. Queued / direct, us: 8 nodes (the 36-triangle box), a million rays any-hit 167 / 112, closest 198 / 175,
+    // 65536 rays 42 / 38, 48 / 44; 14 nodes (168 triangles), a million 130 / 122, 159 / 162, 65536 42 / 40, 50 / 46; from
+    // some 500 nodes on the queue wins (591: 179 / 190 any-hit, 33423: 226 / 237), 50 nodes are even (136 / 138).
+    const bool direct = scene.num_nodes <= kFewNodes;
+    auto launch = [&](auto *queued, auto *tested) {
+        (direct ? tested : queued)<<<g, 128, 0, stream>>>(scene, rays, n, h, counters);
+    };
     if (mode == kTraceClosest) {
         if (count) {
-            k_trace<kTraceClosest, true><<<g, 128, 0, stream>>>(scene, rays, n, h, counters);
+            launch(k_trace<kTraceClosest, true, false>, k_trace<kTraceClosest, true, true>);
         } else {
-            k_trace<kTraceClosest, false><<<g, 128, 0, stream>>>(scene, rays, n, h, counters);
+            launch(k_trace<kTraceClosest, false, false>, k_trace<kTraceClosest, false, true>);
         }
     } else {
         if (count) {
-            k_trace<kTraceAnyRef, true><<<g, 128, 0, stream>>>(scene, rays, n, h, counters);
+            launch(k_trace<kTraceAnyRef, true, false>, k_trace<kTraceAnyRef, true, true>);
         } else {
-            k_trace<kTraceAnyRef, false><<<g, 128, 0, stream>>>(scene, rays, n, h, counters);
+            launch(k_trace<kTraceAnyRef, false, false>, k_trace<kTraceAnyRef, false, true>);
         }
     }
     if (ev) ev->after(stream);

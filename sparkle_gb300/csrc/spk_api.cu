@@ -860,7 +860,7 @@ spk_status upload_scene(spk_ctx *ctx, const HostScene &hs, const std::vector<Dev
     for (int c = 0; c < 3; ++c) S.sky_color[c] = v.sky_color[c];
     S.num_lights = v.num_lights;
     S.light_total = v.light_total;
-    ctx->bvh_nodes = static_cast<uint32_t>(hs.nodes.size());
+    ctx->bvh_nodes = S.num_nodes = static_cast<uint32_t>(hs.nodes.size());
     ctx->bvh_bytes = hs.nodes.size() * sizeof(WideNode) + hs.tris.size() * sizeof(float4);
     ctx->has_scene = true;
     ctx->dirty = true;
@@ -951,7 +951,7 @@ spk_status rebuild_top(spk_ctx *ctx) {
         S.box_lo[a] = ok ? lo[a] : 0.f;
         S.box_scale[a] = ok ? 8.f / (hi[a] - lo[a]) : 0.f;
     }
-    ctx->bvh_nodes = static_cast<uint32_t>(need);
+    ctx->bvh_nodes = S.num_nodes = static_cast<uint32_t>(need);
     ctx->dirty = true;  // any primitive change clears the accumulation (SceneRenderProxy.cpp:198-202)
     return SPK_OK;
 }

@@ -64,6 +64,7 @@ enum : uint32_t { kErrStackOverflow = 1u, kErrIterationBudget = 2u, kErrQueueOve
 #define SPK_PACKET_SIBLINGS 4  // sibling nodes a packet tests at once (one per 8-lane group), 1..4
 #endif
 constexpr int kStackSize = 48;
+constexpr uint32_t kFewNodes = 16;  // scenes of at most this many nodes (TLAS and BLASes) have short walks (launch_trace)
 constexpr int kWalkThreads = 128;  // threads per block of every persistent walking kernel
 constexpr uint32_t kMaxIterations = 1u << 20;
 constexpr uint32_t kPacketSiblings = SPK_PACKET_SIBLINGS;
@@ -435,6 +436,24 @@ struct Walker {
         return false;
     }
 
+    // Tests the triangles of a group at once. True: a hit ends the walk.
+    __device__ __forceinline__ bool test(const DevScene &S, uint2 tg) {
+        for (; tg.y != 0u; tg.y &= tg.y - 1u) {
+            float t, u, v;
+            uint32_t face;
+            if (!triangle_hit(S.tris, tg.x + __ffs(tg.y) - 1, ray, t, u, v, face)) continue;
+            if (kMode == kTraceAnyRef || (kMode == kTraceOcclusion && t < tmax_box)) {
+                best_inst = cur_inst;
+                return true;
+            }
+            if (kMode == kTraceOcclusion) continue;
+            const f3 wo = st.o(), wd = st.d();
+            const float wt = world_t(S.instances[cur_inst], ray, t, wo, wd);
+            if (wt > 0.f && take(wt, u, v, cur_inst, face)) tmax_box = prune_limit(wt, wo.x, wd.x, S.scene_abs_x);
+        }
+        return false;
+    }
+
     // `leaves(item_base, slots, meta)` and `group(tgroup)` take the triangles of the leaf slots reached in a node, and
     // of a group that came back from the stack; either returns true when a hit ends the walk.
     template <class Stack, class Leaves, class Group>
@@ -491,23 +510,7 @@ __device__ __forceinline__ TraceResult trace_ray(const DevScene &S, f3 wo, f3 wd
     LocalStack stack;
     Walker<kMode, kCount, RegState> w;
     w.init(S, S.tlas_root, wo, wd, tmax_occl);
-    auto group = [&](uint2 tg) {
-        while (tg.y != 0u) {
-            const uint32_t idx = tg.x + __ffs(tg.y) - 1;
-            tg.y &= tg.y - 1u;
-            float t, u, v;
-            uint32_t face;
-            if (!triangle_hit(S.tris, idx, w.ray, t, u, v, face)) continue;
-            if (kMode == kTraceAnyRef || (kMode == kTraceOcclusion && t < tmax_occl)) {
-                w.best_inst = w.cur_inst;
-                return true;
-            }
-            if (kMode == kTraceOcclusion) continue;
-            const float wt = world_t(S.instances[w.cur_inst], w.ray, t, wo, wd);
-            if (wt > 0.f && w.take(wt, u, v, w.cur_inst, face)) w.tmax_box = prune_limit(wt, wo.x, wd.x, S.scene_abs_x);
-        }
-        return false;
-    };
+    auto group = [&](uint2 tg) { return w.test(S, tg); };
     auto leaves = [&](uint32_t base, uint32_t slots, const uint32_t (&meta)[2]) {
         return group(make_uint2(base, leaf_items(slots, meta)));
     };
@@ -543,10 +546,11 @@ struct TriangleQueue {
 // store their results, and idle lanes are refilled (22: 16 and 26 are 2% slower). 72 registers (7 blocks per SM) hold a
 // walk without touching local memory in the node visits; more state in shared memory instead (8 blocks) takes L1 from
 // the nodes: measured even.
+// `kDirect`: nothing is queued, a lane tests the triangles of a leaf when it reaches it (launch_trace says when).
 constexpr int kRefillLanes = SPK_REFILL_LANES;
 constexpr uint32_t kTailSteps = SPK_TAIL_STEPS;
 
-template <int kMode, bool kCount, class Fetch, class Finish>
+template <int kMode, bool kCount, bool kDirect, class Fetch, class Finish>
 __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long long *cursor, unsigned long long n,
                                                 float tmax, uint32_t &err, TraceCounts *counts, Fetch &&fetch,
                                                 Finish &&finish) {
@@ -600,6 +604,17 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
             tg.y &= tg.y - 1u;
         }
         return false;
+    };
+    auto test_group = [&](uint2 tg) { return w.test(S, tg); };
+    auto test_leaves = [&](uint32_t base, uint32_t slots, const uint32_t (&meta)[2]) {
+        return w.test(S, make_uint2(base, leaf_items(slots, meta)));
+    };
+    auto step = [&] {
+        if constexpr (kDirect) {
+            return w.step(S, stack, err, counts, test_leaves, test_group);
+        } else {
+            return w.step(S, stack, err, counts, leaves, group);
+        }
     };
     // One round: lane i tests pair i (of `cnt`); hits go to their owners; the pairs past 32 move to the front.
     auto round = [&](uint32_t cnt) {
@@ -698,7 +713,7 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
             continue;
         }
         for (;;) {
-            if (walking && w.step(S, stack, err, counts, leaves, group)) {
+            if (walking && step()) {
                 walking = false;
                 over = true;
             }
@@ -708,7 +723,7 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
             // out of most steps of the last, longest walks (418 rays in host memory: 98 us a call before the queue,
             // 103 with a round every step, 88 with one every 4; 8 the same).
             const bool drain = !exhausted ? walkers < kRefillLanes : walkers == 0u || (++tail_steps % kTailSteps) == 0u;
-            for (;;) {
+            while (!kDirect) {  // (direct: nothing is queued)
                 const uint32_t cnt = min(__shfl_sync(kAll, Q.count, 0), kQueueCap);
                 if (cnt < 32u && !(drain && cnt != 0u)) break;
                 round(cnt);
@@ -910,7 +925,7 @@ __device__ __noinline__ uint32_t walk_wide(const DevScene &S, unsigned long long
 }
 
 // The walk of a launch's rays: one per warp while there are few, else persistent warps with a ray per lane.
-template <int kMode, bool kCount, class Fetch, class Finish>
+template <int kMode, bool kCount, bool kDirect = false, class Fetch, class Finish>
 __device__ __forceinline__ void walk_rays(const DevScene &S, unsigned long long *cursor, unsigned long long n,
                                           float tmax, uint32_t &err, TraceCounts *counts, Fetch &&fetch,
                                           Finish &&finish) {
@@ -919,7 +934,7 @@ __device__ __forceinline__ void walk_rays(const DevScene &S, unsigned long long 
         err |= walk_wide<kMode, kCount>(S, cursor, n, tmax, kCount ? &c : nullptr, fetch, finish);
         if (kCount) *counts = c;
     } else {
-        walk_persistent<kMode, kCount>(S, cursor, n, tmax, err, counts, fetch, finish);
+        walk_persistent<kMode, kCount, kDirect>(S, cursor, n, tmax, err, counts, fetch, finish);
     }
 }
 

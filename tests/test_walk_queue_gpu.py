@@ -107,3 +107,31 @@ def test_any_hit_over_stacked_triangles_is_the_oracles(layers, count):
     assert ctx.stats()["error_flags"] == 0
     assert np.array_equal(got["prim"] != INVALID, hit)
     ctx.close()
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+@pytest.mark.parametrize("count", [33, 8512, 8513, 12769, 34047, 34049, 200_000])
+def test_scenes_of_few_nodes(count, any_hit):
+    """The box (8 instances of few triangles each), whose walks test triangles as they reach them, at ray counts on both
+    sides of where the walks and the grid change: the same as the same rays in launches of 4096, which walk one per
+    warp, and the oracle's hits (a ray that grazes an edge may differ: 2 in 4096, as the smoke test has it)."""
+    scene, _ = scenes.cornell_box(0)
+    rays = scenes.random_rays(*scene.world_bounds(), count, seed=count)
+    ctx = native.Context(0)
+    ctx.set_scene(scene)
+    assert len(ctx.bvh_nodes()) <= 16
+    got = ctx.trace(rays, any_hit=any_hit)
+    st = ctx.stats()
+    assert st["error_flags"] == 0 and st["extension_rays"] == count
+    parts = np.concatenate([ctx.trace(rays[a:a + 4096], any_hit=any_hit) for a in range(0, count, 4096)])
+    ctx.close()
+    ref_scene = oracle.OracleScene(scene)
+    if any_hit:
+        assert np.array_equal(got["prim"] != INVALID, parts["prim"] != INVALID)
+        want, _ = ref_scene.trace(rays, any_hit=True)
+        wrong = int(((got["prim"] != INVALID) != (want["prim"] != INVALID)).sum())
+    else:
+        assert got.tobytes() == parts.tobytes()
+        c = classify_hits(got, oracle_hits(ref_scene, rays, oracle.PRUNED)[0])
+        wrong = count - c["exact"] - c["tie"]
+    assert wrong <= max(2, count // 2048)
