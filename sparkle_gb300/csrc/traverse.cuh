@@ -34,7 +34,7 @@ enum : uint32_t { kErrStackOverflow = 1u, kErrIterationBudget = 2u, kErrQueueOve
 #define SPK_REFILL_LANES 22  // persistent warps refill idle lanes once fewer than this are walking
 #endif
 #ifndef SPK_WIDE_RAYS_PER_BLOCK
-#define SPK_WIDE_RAYS_PER_BLOCK 12  // launches of at most this many rays per block walk one ray per warp
+#define SPK_WIDE_RAYS_PER_BLOCK 12  // launches of at most this many rays per block walk one ray per warp (walk_rays)
 #endif
 #ifndef SPK_TAIL_STEPS
 #define SPK_TAIL_STEPS 4  // steps between the rounds of a persistent warp that has no more rays to fetch
@@ -745,8 +745,10 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
 // visits one node. Same boxes (the plain slab test with a correctly rounded reciprocal), triangles and tie rule, so the
 // same results. `fetch` and `finish` as for walk_persistent; `finish` runs in one lane.
 // 4097 rays: 49 -> 22 us (11392 triangles). It takes 6 times the instructions per ray, so more rays soon do better with
-// a ray per lane: up to 12 rays per block (12768 on 152 SMs) it won or tied on all scenes, at 16 the 36-triangle box lost
-// 6% (its walks are short), at 8 a 10627-ray query of 200480 triangles took 117 us instead of 102.
+// a ray per lane: beyond 12 rays per block (12768 on 152 SMs), or, in scenes of few nodes, whose walks are over in a few steps,
+// 5/8 of the nodes, at least 4. One per warp / per lane, us a closest-hit query: 12768 rays of 1188, 33423 and 312823
+// nodes 58 / 69, 62 / 78, 71 / 100; of 13 nodes 5320 rays 32 / 34, 8512 rays 36 / 36, 12768 rays 40 / 36; of 8 nodes 4097
+// rays 35 / 35, 6385 rays 40 / 36, 12768 rays 52 / 38.
 constexpr int kWideStack = 96;  // a step pushes at most 8 groups
 // Not inlined, so that its registers do not count against walk_persistent's in the same kernel. Returns error bits.
 template <int kMode, bool kCount, class Fetch, class Finish>
@@ -929,7 +931,8 @@ template <int kMode, bool kCount, bool kDirect = false, class Fetch, class Finis
 __device__ __forceinline__ void walk_rays(const DevScene &S, unsigned long long *cursor, unsigned long long n,
                                           float tmax, uint32_t &err, TraceCounts *counts, Fetch &&fetch,
                                           Finish &&finish) {
-    if (n <= static_cast<unsigned long long>(gridDim.x) * SPK_WIDE_RAYS_PER_BLOCK) {
+    const uint32_t per_block = max(4u, min(static_cast<uint32_t>(SPK_WIDE_RAYS_PER_BLOCK), min(S.num_nodes, 64u) * 5u / 8u));
+    if (n <= static_cast<unsigned long long>(gridDim.x) * per_block) {
         TraceCounts c;
         err |= walk_wide<kMode, kCount>(S, cursor, n, tmax, kCount ? &c : nullptr, fetch, finish);
         if (kCount) *counts = c;
