@@ -253,3 +253,32 @@ def test_identity_refit_ranges(ctx, side, scale, offset):
     before = ctx.bvh_nodes()
     ctx.update_mesh(0, pos)
     assert np.array_equal(before, ctx.bvh_nodes())
+
+
+@pytest.mark.parametrize("side", [1, 64, 65])
+def test_moved_mesh_bounds(ctx, side):
+    """2, 8192 and 8450 faces (up to 8192 the host takes the mesh's new box, above it comes from the refitted root),
+    moved out of the box the mesh had: hits as in a context built from the moved mesh."""
+    x, y = np.meshgrid(np.linspace(-3, 3, side + 1), np.linspace(-3, 3, side + 1), indexing="ij")
+    pos = np.stack([x, y, 0.3 * np.sin(x + 2 * y)], -1).reshape(-1, 3).astype(np.float32)
+    a = (np.arange(side)[:, None] * (side + 1) + np.arange(side)[None, :]).reshape(-1)
+    faces = np.concatenate([np.stack([a, a + side + 1, a + 1], 1), np.stack([a + 1, a + side + 1, a + side + 2], 1)])
+    moved_pos = pos * np.float32([1.5, 0.5, 2.0]) + np.float32([20.0, -7.0, 3.0])
+
+    def scene_of(p):
+        scene, _ = copy.deepcopy(scenes.cornell_box(0))
+        mesh = scene.meshes[0]
+        mesh.positions, mesh.indices = p, faces.astype(np.uint32)
+        mesh.normals, mesh.tangents, mesh.uvs = np.tile(np.float32([0, 0, 1]), (len(p), 1)), None, None
+        return scene
+
+    moved = scene_of(moved_pos)
+    rays = scenes.random_rays(moved_pos.min(0) - 2, moved_pos.max(0) + 2, 20_000, seed=side)
+    fresh = native.Context(0)
+    fresh.set_scene(moved)
+    ref = fresh.trace(rays)
+    fresh.close()
+    ctx.set_scene(scene_of(pos))
+    ctx.update_mesh(0, moved_pos)
+    hits_equal(ctx.trace(rays), ref)
+    assert (ref["prim"] != 0xFFFFFFFF).mean() > 0.1
