@@ -33,11 +33,10 @@ constexpr int kPacketQueue = 8;
 constexpr int kPacket2Queue = 9;
 constexpr int kNextItem = 10;  // next (frame, pixel) sample item to hand out
 
-// A walk's grid fills the SMs and spreads evenly however its blocks come in (chained_launch.cuh); the shading grids do
-// not, and shading many paths from uneven places costs more than the launch, so a walk of more than kEarlyRays rays
-// lets them in as its last blocks leave (1080p, 64 samples: 101.07 ms with all let in early, 100.63 so, 100.78 with
-// plain launches; 335 x 202, 1 sample: 494, 492 and 552 us with an event node on each side of the walks).
-constexpr unsigned long long kEarlyRays = 1ull << 20;
+// The shading stages let the next kernel in as they start (chained_launch.cuh). A walk does not: the kernel behind it
+// comes in as its blocks leave. Let in with the walk's start it waits beside it and takes part of the SMs: us without /
+// with, 335 x 202 at one sample of the 3.4M-triangle scene 727 / 736, 1080p 3016 / 3040, 853 x 481 with light sampling
+// 4770 / 4816, the box at 256 x 256 246 / 261, 1080p at 64 samples 107110 / 107487.
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -279,7 +278,6 @@ __global__ void __launch_bounds__(128, kPackets == 2   ? SPK_PACKET2_MIN_BLOCKS
     const unsigned long long p2 = min(counters->queue_counters[kPacket2Queue], p1);
     const unsigned long long first = kPackets == 2 ? 0ull : kPackets == 1 ? p2 : p1;
     const unsigned long long n = (kPackets == 2 ? p2 : kPackets == 1 ? p1 : len) - first;
-    if (n <= kEarlyRays) let_next_kernel_in();
     if (n == 0) return;
     uint32_t err = 0;
     TraceCounts tc;
@@ -842,7 +840,6 @@ __global__ void __launch_bounds__(128, SPK_SHADOW_MIN_BLOCKS) k_wf_shadow(const 
     after_previous_kernel();
     uint32_t err = 0;
     const unsigned long long n = counters->queue_counters[kShadowLen];
-    if (n <= kEarlyRays) let_next_kernel_in();
     walk_rays<kTraceOcclusion, false>(
         S, &counters->queue_counters[kShadowCursor], n, kFltMax, err, nullptr,
         [&S, &s](unsigned long long q, f3 &o, f3 &d, float &tmax) {
