@@ -135,3 +135,32 @@ def test_scenes_of_few_nodes(count, any_hit):
         c = classify_hits(got, oracle_hits(ref_scene, rays, oracle.PRUNED)[0])
         wrong = count - c["exact"] - c["tie"]
     assert wrong <= max(2, count // 2048)
+
+
+def test_edge_rays_one_per_warp():
+    """Rays that leave the box from a point of its walls, nearly along them (their hits are decided by the last bit), in
+    launches of 4096, which walk one ray per warp there, against one launch of all."""
+    scene, _ = scenes.cornell_box(0)
+    lo, hi = (np.asarray(v, np.float32) for v in scene.world_bounds())
+    rng = np.random.default_rng(11)
+    n = 65_536
+    axis, rows = rng.integers(0, 3, n), np.arange(n)
+    side = rng.integers(0, 2, n) == 1
+    near = (axis + 1) % 3
+    o = (lo + (hi - lo) * rng.random((n, 3))).astype(np.float32)
+    o[rows, axis] = np.where(side, hi[axis], lo[axis])
+    o[rows, near] = (lo[near] + (hi[near] - lo[near]) * 10 ** rng.uniform(-6, -2, n)).astype(np.float32)
+    d = rng.standard_normal((n, 3))
+    d[rows, axis] = np.where(side, 1, -1) * 10 ** rng.uniform(-7, -2, n)
+    d[rows, near] = -np.abs(d[rows, near])
+    rays = abi.rays_to_array(o, d / np.linalg.norm(d, axis=1, keepdims=True))
+    ctx = native.Context(0)
+    ctx.set_scene(scene)
+    for any_hit in (False, True):
+        whole = ctx.trace(rays, any_hit=any_hit)
+        parts = np.concatenate([ctx.trace(rays[a:a + 4096], any_hit=any_hit) for a in range(0, n, 4096)])
+        if any_hit:
+            assert np.array_equal(whole["prim"] != INVALID, parts["prim"] != INVALID)
+        else:
+            assert whole.tobytes() == parts.tobytes()
+    ctx.close()
