@@ -106,9 +106,9 @@ __device__ void quantize(NodeBytes &n, const float clo[8][3], const float chi[8]
 
 // One axis of a node, quantised as quantize() does it, by the eight lanes of the node (each with its own slot's
 // box [cl, ch]; empty slots hold anything). In float: the difference to the origin is rounded to d with the exact
-// error e, d times a power of two is exact, and rounding is monotone, so d compares with an integer as the exact
-// difference does unless d is that integer and e is not 0. Those lanes, and axes outside the range where no
-// intermediate result over- or underflows, take quantize()'s doubles.
+// error e (Knuth's two-sum, The Art of Computer Programming 2, 4.2.2), d times a power of two is exact, and rounding
+// is monotone, so d compares with an integer as the exact difference does unless d is that integer and e is not 0.
+// Those lanes, and axes outside the range where no intermediate result over- or underflows, take quantize()'s doubles.
 struct AxisBytes {
     uint32_t exponent, lo, hi;
 };

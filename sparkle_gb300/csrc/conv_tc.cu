@@ -319,10 +319,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 // K blocks, row taps and half chunks run in k_conv_fwd's order: the sums are the same bit for bit.
 // What k_conv_fwd spends most of a narrow layer on is each CTA's set-up, first load and epilogue, one after the
 // other: without any MMA a 32 -> 32 layer of 1920 x 1088 took 82 of its 88 us. Here they overlap: 59 us, 4.5
-// TB/s of input and output. What is left is mostly the MMAs' reads of A (128 rows of 32 bytes for 32 columns
-// of output, about 55 cycles each). 64 -> 64 at 960 x 544: 54.7 -> 37.9 us. Input boxes stored once per chunk
-// as planes without swizzle, where all nine taps are start addresses, were slower (91 us): the MMA reads such
-// a box at about 80 cycles each.
+// TB/s of input and output. What is left is shared memory: by the counters its data pipe is taken 63% by the MMAs'
+// operands (128 rows of A for 32 columns of output) and 38% by the epilogue's staging, the tensor pipe 30%, DRAM 43%.
+// 64 -> 64 at 960 x 544: 54.7 -> 37.9 us. Input boxes stored once per chunk as planes without swizzle, where all nine
+// taps are start addresses, were slower (91 us).
 constexpr uint32_t kResTile = 16;  // tile side
 constexpr uint32_t kResM = 2;      // M tiles
 constexpr uint32_t kResMRows = kResTile / kResM;

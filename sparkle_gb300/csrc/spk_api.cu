@@ -1900,8 +1900,9 @@ spk_status spk_trace(spk_ctx *ctx, const spk_ray *rays, uint64_t num_rays, spk_h
     if (!ctx->has_scene) return fail(ctx, SPK_ERR_NOT_READY, "trace needs spk_set_scene first");
     cudaSetDevice(ctx->device);
     if (num_rays == 0) return SPK_OK;
-    // Rays, then hits, in one device buffer that the context keeps between calls (allocating and freeing it took
-    // a third of larger ones and a sixth of small ones: 71111 rays 381 -> 221 us, 4097 rays 85 -> 72 us); a buffer above kTraceKeep is given back at the end of the call.
+    // Rays, then hits, in one device buffer that the context keeps between calls (allocating and freeing it took a third
+    // of larger ones and a sixth of small ones: 71111 rays 381 -> 221 us, 4097 rays 85 -> 72 us); a buffer above
+    // kTraceKeep is given back at the end of the call.
     cudaError_t e;
     const size_t ray_bytes = (num_rays * sizeof(spk_ray) + 255) / 256 * 256;
     const size_t bytes = ray_bytes + num_rays * sizeof(spk_hit);

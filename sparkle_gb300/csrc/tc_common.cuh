@@ -183,9 +183,8 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by the lane with `issue` set. The whole warp calls it with the same
-// operands, outside divergent code: the descriptors, given as (low, high) words, then stay in uniform
-// registers, where the instruction takes them from. Under `lane == 0` each MMA first had its operands moved
-// there one by one (forward 32 -> 32 at 1920 x 1088: 95 us, now 88; 96 -> 32: 184, now 174).
+// operands, given as (low, high) descriptor words, outside divergent code (forward 32 -> 32 at 1920 x 1088: 95 us
+// under `lane == 0`, 88 so; 96 -> 32: 184 and 174).
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                          uint32_t idesc, uint32_t accumulate, bool issue) {
     asm volatile(

@@ -522,9 +522,10 @@ __device__ __forceinline__ TraceResult trace_ray(const DevScene &S, f3 wo, f3 wd
 // The triangles a warp's rays have reached and not tested yet: (triangle, instance) pairs with the lane that owns
 // the ray. Tested in the lane that reached them, triangles ran at 3.2 of 32 lanes (secondary rays of the 1024^2
 // terrain: 2 warp executions per ray, 30% of the walk's instructions); queued, a round tests 32 pairs with 26 lanes on
-// average: 550 -> 400 warp instructions per ray over the whole walk. Queueing groups instead of triangles saves the
-// writes but costs a scan per round (+4% instructions).
-constexpr uint32_t kQueueCap = 64;  // a round leaves fewer than 32, a step adds about 8 (what does not fit goes to the stack)
+// average. With this and the packed slab tests bounces 1 to 7 of a 64-sample 1080p frame went from 523 to 444 warp
+// instructions per ray. Queueing groups instead of triangles saves the writes but costs a scan per round (+4%
+// instructions).
+constexpr uint32_t kQueueCap = 64;  // a round leaves fewer than 32, a step adds about 8 (the rest goes to the stack)
 struct TriangleQueue {
     uint2 pair[kQueueCap];      // triangle record, instance
     uint8_t owner[kQueueCap];
@@ -543,7 +544,7 @@ struct TriangleQueue {
 // pair's instance space (the same operations as at the BLAS entry, so the same bits). A hit goes back to its
 // owner, whose best t then prunes as before: a few steps later than if tested at once, which adds node visits (+1.6%)
 // but cannot change a result. When fewer than kRefillLanes lanes walk, every pair is tested, the walks that are over
-// store their results, and idle lanes are refilled (22: 16 and 26 are 2% slower). 72 registers (7 blocks per SM) hold a
+// store their results, and idle lanes are refilled (22: 16 and 26 are 0.6 and 1.6% slower on a 64-sample 1080p frame). 72 registers (7 blocks per SM) hold a
 // walk without touching local memory in the node visits; more state in shared memory instead (8 blocks) takes L1 from
 // the nodes: measured even.
 // `kDirect`: nothing is queued, a lane tests the triangles of a leaf when it reaches it (launch_trace says when).
@@ -720,8 +721,9 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
             __syncwarp();
             const uint32_t walkers = __popc(__ballot_sync(kAll, walking));
             // Once the list is exhausted there is nothing to refill: every few steps, which keeps a round's latency
-            // out of most steps of the last, longest walks (418 rays in host memory: 98 us a call before the queue,
-            // 103 with a round every step, 88 with one every 4; 8 the same).
+            // out of most steps of the last, longest walks (a round every 1 / 4 / 8 / 16 steps, us: 65536 rays of the
+            // 3.4M-triangle scene 140 / 129 / 129 / 135, 12769 of 11392 triangles 72 / 68 / 69 / 68, a 1080p frame of one
+            // sample 3076 / 3044 / 3034 / 3054).
             const bool drain = !exhausted ? walkers < kRefillLanes : walkers == 0u || (++tail_steps % kTailSteps) == 0u;
             while (!kDirect) {  // (direct: nothing is queued)
                 const uint32_t cnt = min(__shfl_sync(kAll, Q.count, 0), kQueueCap);
@@ -745,8 +747,8 @@ __device__ __forceinline__ void walk_persistent(const DevScene &S, unsigned long
 // visits one node. Same boxes (the plain slab test with a correctly rounded reciprocal), triangles and tie rule, so the
 // same results. `fetch` and `finish` as for walk_persistent; `finish` runs in one lane.
 // 4097 rays: 49 -> 22 us (11392 triangles). It takes 6 times the instructions per ray, so more rays soon do better with
-// a ray per lane: beyond 12 rays per block (12768 on 152 SMs), or, in scenes of few nodes, whose walks are over in a few steps,
-// 5/8 of the nodes, at least 4. One per warp / per lane, us a closest-hit query: 12768 rays of 1188, 33423 and 312823
+// a ray per lane: beyond 12 rays per block (12768 on 152 SMs), or, in scenes of few nodes, whose walks are over in a
+// few steps, 5/8 of the nodes, at least 4. One per warp / per lane, us a closest-hit query: 12768 rays of 1188, 33423 and 312823
 // nodes 58 / 69, 62 / 78, 71 / 100; of 13 nodes 5320 rays 32 / 34, 8512 rays 36 / 36, 12768 rays 40 / 36; of 8 nodes 4097
 // rays 35 / 35, 6385 rays 40 / 36, 12768 rays 52 / 38.
 constexpr int kWideStack = 96;  // a step pushes at most 8 groups

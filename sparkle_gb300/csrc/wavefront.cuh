@@ -38,7 +38,6 @@ struct WavefrontState {
     size_t sample_capacity = 0;               // float4 entries of `samples`
     float4 *sample_normals = nullptr;         // multi-frame mode with the spatial fill: first-hit normal per sample
     size_t normal_capacity = 0;               // float4 entries of `sample_normals`
-    // multi-frame mode: per-frame constants, frame k of the call
     unsigned long long *host_len = nullptr;  // pinned: queue length read back between iteration chunks
     // Shadow stage of next-event estimation (allocated on first use, `nee_capacity` slots): the two
     // occlusion rays of a light-sampling vertex (k = 0 light, 1 sky) and the radiance each adds unoccluded.
@@ -79,8 +78,8 @@ struct WfTuning {
 // Allocates the shadow-stage buffers of `s` for its capacity (no-op when they are large enough).
 cudaError_t wavefront_alloc_nee(WavefrontState &s);
 
-// Host-side CUDA graph of one chunk of the multi-frame loop (kChunkIterations extend + shade iterations
-// with their counter resets), captured once and replayed while the kernel parameters stay the same.
+// Host-side CUDA graph of one chunk of the multi-frame loop (up to kChunkIterations extend + shade iterations),
+// captured once and replayed while the kernel parameters stay the same.
 constexpr uint32_t kChunkIterations = 8;
 struct ChunkGraph {
     cudaGraphExec_t exec = nullptr;
