@@ -348,7 +348,8 @@ spk_status spk_get_config(const spk_ctx *ctx, spk_config *out);
  * the clear (if dirty), BasePass (:419-450), DenoisePass (:506-552) and ToneMappingPass (:565-576), with
  * the camera's cumulated-sample bookkeeping between frames (CameraRenderProxy.cpp:66-75). Asynchronous
  * with respect to the host: results are visible to spk_read_framebuffer / spk_synchronize. A call that fails
- * leaves the accumulation as it was; one of more than 64 frames may have folded some and restarts it. */
+ * leaves the accumulation as it was; one of more than 64 frames may have folded some and restarts it, and frame by
+ * frame (spk_tuning.multi_frame = 0, the one-kernel schedule) the frames before the failing one stay folded and counted. */
 spk_status spk_render(spk_ctx *ctx, uint32_t num_frames);
 
 /* Copies the accumulated HDR frame buffer (`frame_buffer_`, H rows of W float4, row j = image row j from
